@@ -402,7 +402,7 @@ int ensure_proposal_state(bafqmc_handle* h) {
     CK(cudaMalloc(&h->d_arena2, sizeof(double2) * h->arena_total));
     CK(cudaMalloc(&h->d_phi2, sizeof(double) * h->phi_total));
     CK(cudaMalloc(&h->d_sc2, sizeof(ChainScalars) * h->nchains));
-    CK(cudaMemset(h->d_sc2, 0, sizeof(ChainScalars) * h->nchains));
+    CK(cudaMemsetAsync(h->d_sc2, 0, sizeof(ChainScalars) * h->nchains, h->stream));
     CK(cudaMalloc(&h->d_fn2, sizeof(double) * h->nchains));
     CK(cudaMalloc(&h->d_acc, sizeof(int) * h->nchains));
     return BAFQMC_OK;
@@ -569,11 +569,18 @@ int bafqmc_create_tuned(const bafqmc_point* pts, int npts, const int32_t* chain_
         return bail(e, "upload pstart");
     if ((e = cudaMemcpy(h->d_plist, plist.data(), sizeof(int) * nchains, cudaMemcpyHostToDevice)) != cudaSuccess)
         return bail(e, "upload plist");
-    if ((e = cudaMemset(h->d_arena, 0, sizeof(double2) * h->arena_total)) != cudaSuccess) return bail(e, "memset arena");
-    if ((e = cudaMemset(h->d_obs, 0, sizeof(double) * (size_t)nchains * h->obs_stride)) != cudaSuccess)
+    // Cleared on the handle's stream: it does not wait for the legacy stream, where the clearing
+    // (milliseconds for an arena of GBs) could overtake the state that the caller uploads next.
+    if ((e = cudaMemsetAsync(h->d_arena, 0, sizeof(double2) * h->arena_total, h->stream)) != cudaSuccess)
+        return bail(e, "memset arena");
+    if ((e = cudaMemsetAsync(h->d_obs, 0, sizeof(double) * (size_t)nchains * h->obs_stride, h->stream)) != cudaSuccess)
         return bail(e, "memset obs");
-    if ((e = cudaMemset(h->d_sc, 0, sizeof(ChainScalars) * nchains)) != cudaSuccess) return bail(e, "memset sc");
-    if ((e = cudaMemset(h->d_phi, 0, sizeof(double) * h->phi_total)) != cudaSuccess) return bail(e, "memset phi");
+    if ((e = cudaMemsetAsync(h->d_sc, 0, sizeof(ChainScalars) * nchains, h->stream)) != cudaSuccess)
+        return bail(e, "memset sc");
+    if ((e = cudaMemsetAsync(h->d_phi, 0, sizeof(double) * h->phi_total, h->stream)) != cudaSuccess)
+        return bail(e, "memset phi");
+    // the tables above were copied on the legacy stream, from pageable memory
+    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return bail(e, "upload tables");
     *out = h;
     return BAFQMC_OK;
 }
@@ -1124,7 +1131,8 @@ int bafqmc_set_time_displaced(bafqmc_handle* h, int enable, int probe_nt) {
         for (int c = 0; c < h->nchains; ++c) idx[c] = c;
         int* p = nullptr;
         CK(cudaMalloc(&p, sizeof(int) * h->nchains));
-        const cudaError_t e = cudaMemcpy(p, idx.data(), sizeof(int) * h->nchains, cudaMemcpyHostToDevice);
+        const cudaError_t e =
+            cudaMemcpyAsync(p, idx.data(), sizeof(int) * h->nchains, cudaMemcpyHostToDevice, h->stream);
         if (e != cudaSuccess) {
             cudaFree(p);
             return cuda_fail(e, "chain list of the time-displaced pass");
@@ -1135,7 +1143,7 @@ int bafqmc_set_time_displaced(bafqmc_handle* h, int enable, int probe_nt) {
     if (!h->d_tau_stats) {
         double* p = nullptr;
         CK(cudaMalloc(&p, sizeof(double) * bq::kTauStats * h->nchains));
-        const cudaError_t e = cudaMemset(p, 0, sizeof(double) * bq::kTauStats * h->nchains);
+        const cudaError_t e = cudaMemsetAsync(p, 0, sizeof(double) * bq::kTauStats * h->nchains, h->stream);
         if (e != cudaSuccess) {
             cudaFree(p);
             return cuda_fail(e, "drift statistics of the time-displaced pass");
@@ -1145,7 +1153,7 @@ int bafqmc_set_time_displaced(bafqmc_handle* h, int enable, int probe_nt) {
     if (probe_nt > 0 && !h->d_tau_probe) {
         double2* p = nullptr;
         CK(cudaMalloc(&p, sizeof(double2) * bq::kTauProbeElems * h->nchains));
-        const cudaError_t e = cudaMemset(p, 0, sizeof(double2) * bq::kTauProbeElems * h->nchains);
+        const cudaError_t e = cudaMemsetAsync(p, 0, sizeof(double2) * bq::kTauProbeElems * h->nchains, h->stream);
         if (e != cudaSuccess) {
             cudaFree(p);
             return cuda_fail(e, "probe of the time-displaced pass");

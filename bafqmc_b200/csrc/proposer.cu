@@ -751,7 +751,9 @@ int upload_configs(bafqmc_net* n, int count, const double* a, const double* b) {
     for (long long k = 0; k < per * count; ++k) h[k] = (float)a[k];
     if (b)
         for (long long k = 0; k < per * count; ++k) h[per * count + k] = (float)b[k];
-    NCK(cudaMemcpy(n->d_tin, h.data(), sizeof(float) * need, cudaMemcpyHostToDevice));
+    // on the network's stream, which does not wait for a copy on the legacy stream
+    NCK(cudaMemcpyAsync(n->d_tin, h.data(), sizeof(float) * need, cudaMemcpyHostToDevice, n->stream));
+    NCK(cudaStreamSynchronize(n->stream));
     return BAFQMC_OK;
 }
 
@@ -804,13 +806,13 @@ int bafqmc_net_create(int Lx, int Ly, int Ltrot, int width, int device, bafqmc_n
     }
     float** bufs[] = {&n->d_params, &n->d_grad, &n->d_adam_m, &n->d_adam_v, &n->d_wq};
     for (float** b : bufs) {
-        if (cudaMalloc(b, np) != cudaSuccess || cudaMemset(*b, 0, np) != cudaSuccess)
+        if (cudaMalloc(b, np) != cudaSuccess || cudaMemsetAsync(*b, 0, np, n->stream) != cudaSuccess)
             return bail(bq::net_fail(BAFQMC_ECUDA, "cudaMalloc parameters"));
     }
     if (cudaMalloc(&n->d_wt, sizeof(__nv_bfloat16) * wt) != cudaSuccess ||
-        cudaMemset(n->d_wt, 0, sizeof(__nv_bfloat16) * wt) != cudaSuccess ||
+        cudaMemsetAsync(n->d_wt, 0, sizeof(__nv_bfloat16) * wt, n->stream) != cudaSuccess ||
         cudaMalloc(&n->d_loss, sizeof(double)) != cudaSuccess || cudaMalloc(&n->d_err, sizeof(int)) != cudaSuccess ||
-        cudaMemset(n->d_err, 0, sizeof(int)) != cudaSuccess)
+        cudaMemsetAsync(n->d_err, 0, sizeof(int), n->stream) != cudaSuccess)
         return bail(bq::net_fail(BAFQMC_ECUDA, "cudaMalloc network state"));
     n->use_tc = bq::conv_tc_applies(s, 1, false) ? 1 : 0;
     *out = n;
@@ -891,7 +893,7 @@ int bafqmc_net_loss_grad(bafqmc_net* n, int chains, const double* phi, const dou
         pairs[b] = b;
         pairs[chains + b] = chains + b;
     }
-    NCK(cudaMemcpy(n->d_pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice));
+    NCK(cudaMemcpyAsync(n->d_pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice, n->stream));
     NCK(bq::launch_pack_data(n, n->d_tin, nullptr, chains));
     NCK(bq::net_loss_grad_src(n, chains, n->d_tin));
     if (loss) NCK(cudaMemcpyAsync(loss, n->d_loss, sizeof(double), cudaMemcpyDeviceToHost, n->stream));
@@ -946,7 +948,7 @@ int bafqmc_net_set_wait_test(bafqmc_net* n, int enable) {
     NCK(cudaSetDevice(n->device));
     NCK(cudaStreamSynchronize(n->stream));
     n->wait_test = enable ? 1 : 0;
-    NCK(cudaMemset(n->d_err, 0, sizeof(int)));   // a new test (or its end) starts from a clean status
+    NCK(cudaMemsetAsync(n->d_err, 0, sizeof(int), n->stream));   // a new test (or its end) starts from a clean status
     return BAFQMC_OK;
 }
 
