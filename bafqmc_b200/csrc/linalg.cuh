@@ -13,186 +13,30 @@
 // for the whole sequence and reduce with shuffles, so no step needs a block
 // barrier; divisions are replaced by precomputed reciprocals.
 #pragma once
-#include "cplx.cuh"
+#include "mma64.cuh"
 
 // Factorisation routines are kept out of line: they run once per wrap, and
 // inlining them into the sweep kernel costs registers on the per-slice path.
 #define COLD static __device__ __noinline__
 
-// Strided operand view: element (r, c) = p[r*sr + c*sc], optionally conjugated.
-// A transposed view swaps the strides.  p may point to shared or global memory.
-struct MatOp {
-    const cplx* p;
-    int sr, sc;
-    int cj;
-    DEVI cplx at(int r, int c) const {
-        cplx v = p[(long)r * sr + (long)c * sc];
-        return cj ? cconj(v) : v;
-    }
-};
-DEVI MatOp op_n(const cplx* p, int ld) { return MatOp{p, ld, 1, 0}; }
-DEVI MatOp op_c(const cplx* p, int ld) { return MatOp{p, 1, ld, 1}; }   // conjugate transpose
-
-enum { TRI_NONE = 0, TRI_A_UPPER = 1, TRI_B_LOWER_FROM_C = 2 };
-
-// C = A * B for n x n operands, each thread computing a TR x TC micro-tile.
-// C may alias A or B: results are staged in registers across a barrier.
-// tri = TRI_A_UPPER zeroes A(r,k) for k < r (ZTRMM 'L','U','N');
-// tri = TRI_B_LOWER_FROM_C zeroes B(k,c) for k < c (ZTRMM 'R','U','C').
-template <int TR, int TC>
+// C = A * B for n x n operands (C may alias A or B), the complex product of
+// prod_mma out of line.  tri as there.
+template <int RT, int CT, int RND, bool SH>
 COLD void gemm_rs(int n, int ld, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) {
-    const int ncg = (n + TC - 1) / TC, nrg = (n + TR - 1) / TR;
-    const int g = threadIdx.x;
-    const bool active = g < ncg * nrg;
-    const int r0 = active ? (g / ncg) * TR : 0, c0 = active ? (g % ncg) * TC : 0;
-    cplx acc[TR][TC];
-#pragma unroll
-    for (int i = 0; i < TR; ++i)
-#pragma unroll
-        for (int j = 0; j < TC; ++j) acc[i][j] = cmk(0.0, 0.0);
-    if (active) {
-        for (int k = 0; k < n; ++k) {
-            cplx a[TR], b[TC];
-#pragma unroll
-            for (int i = 0; i < TR; ++i) {
-                int r = r0 + i;
-                a[i] = (r < n) ? A.at(r, k) : cmk(0.0, 0.0);
-                if (tri == TRI_A_UPPER && k < r) a[i] = cmk(0.0, 0.0);
-            }
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-                int c = c0 + j;
-                b[j] = (c < n) ? B.at(k, c) : cmk(0.0, 0.0);
-                if (tri == TRI_B_LOWER_FROM_C && k < c) b[j] = cmk(0.0, 0.0);
-            }
-#pragma unroll
-            for (int i = 0; i < TR; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-        }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-                int r = r0 + i, c = c0 + j;
-                if (r < n && c < n) C[r * ld + c] = acc[i][j];
-            }
-    }
-    __syncthreads();
-}
-
-// C = A * B with A, B, C n x n row-major in shared memory (C may alias A or
-// B); the per-slice propagation products.
-template <int TR, int TC>
-DEVI void gemm_smem(int n, int ld, cplx* C, const cplx* A, const cplx* B) {
-    const int ncg = (n + TC - 1) / TC, nrg = (n + TR - 1) / TR;
-    const int g = threadIdx.x;
-    const bool active = g < ncg * nrg;
-    const int r0 = active ? (g / ncg) * TR : 0, c0 = active ? (g % ncg) * TC : 0;
-    cplx acc[TR][TC];
-#pragma unroll
-    for (int i = 0; i < TR; ++i)
-#pragma unroll
-        for (int j = 0; j < TC; ++j) acc[i][j] = cmk(0.0, 0.0);
-    if (active) {
-        int ra[TR], cb[TC];
-#pragma unroll
-        for (int i = 0; i < TR; ++i) ra[i] = min(r0 + i, n - 1) * ld;
-#pragma unroll
-        for (int j = 0; j < TC; ++j) cb[j] = min(c0 + j, n - 1);
-        for (int k = 0; k < n; ++k) {
-            cplx a[TR], b[TC];
-#pragma unroll
-            for (int i = 0; i < TR; ++i) a[i] = A[ra[i] + k];
-#pragma unroll
-            for (int j = 0; j < TC; ++j) b[j] = B[k * ld + cb[j]];
-#pragma unroll
-            for (int i = 0; i < TR; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-        }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-                const int r = r0 + i, c = c0 + j;
-                if (r < n && c < n) C[r * ld + c] = acc[i][j];
-            }
-    }
-    __syncthreads();
+    prod_mma<RT, CT, RND, PROD_CC, SH>(n, ld, C, A, B, nullptr, tri);
 }
 
 // The slice propagators e^{-+dtau K} are real (real hopping, chemical
 // potential and pairing amplitude), so the per-slice products are complex x
 // real.  Real operands are stored as doubles with the same leading dimension.
-// acc += a * b with real b is (fma(a.x, b, acc.x), fma(a.y, b, acc.y)): the same
-// values as the complex product with a zero imaginary part, in half the FLOPs.
-template <int TR, int TC, bool RIGHT_REAL>
+template <int RT, int CT, int RND, bool RIGHT_REAL, bool SH>
 DEVI void gemm_smem_real(int n, int ld, cplx* C, const void* Ap, const void* Bp) {
-    const int ncg = (n + TC - 1) / TC, nrg = (n + TR - 1) / TR;
-    const int g = threadIdx.x;
-    const bool active = g < ncg * nrg;
-    const int r0 = active ? (g / ncg) * TR : 0, c0 = active ? (g % ncg) * TC : 0;
-    cplx acc[TR][TC];
-#pragma unroll
-    for (int i = 0; i < TR; ++i)
-#pragma unroll
-        for (int j = 0; j < TC; ++j) acc[i][j] = cmk(0.0, 0.0);
-    if (active) {
-        int ra[TR], cb[TC];
-#pragma unroll
-        for (int i = 0; i < TR; ++i) ra[i] = min(r0 + i, n - 1) * ld;
-#pragma unroll
-        for (int j = 0; j < TC; ++j) cb[j] = min(c0 + j, n - 1);
-        for (int k = 0; k < n; ++k) {
-            if (RIGHT_REAL) {   // C = A (complex) * B (real)
-                const cplx* A = static_cast<const cplx*>(Ap);
-                const double* B = static_cast<const double*>(Bp);
-                cplx a[TR];
-                double b[TC];
-#pragma unroll
-                for (int i = 0; i < TR; ++i) a[i] = A[ra[i] + k];
-#pragma unroll
-                for (int j = 0; j < TC; ++j) b[j] = B[k * ld + cb[j]];
-#pragma unroll
-                for (int i = 0; i < TR; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC; ++j)
-                        acc[i][j] = cmk(fma(a[i].x, b[j], acc[i][j].x), fma(a[i].y, b[j], acc[i][j].y));
-            } else {            // C = A (real) * B (complex)
-                const double* A = static_cast<const double*>(Ap);
-                const cplx* B = static_cast<const cplx*>(Bp);
-                double a[TR];
-                cplx b[TC];
-#pragma unroll
-                for (int i = 0; i < TR; ++i) a[i] = A[ra[i] + k];
-#pragma unroll
-                for (int j = 0; j < TC; ++j) b[j] = B[k * ld + cb[j]];
-#pragma unroll
-                for (int i = 0; i < TR; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC; ++j)
-                        acc[i][j] = cmk(fma(a[i], b[j].x, acc[i][j].x), fma(a[i], b[j].y, acc[i][j].y));
-            }
-        }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-                const int r = r0 + i, c = c0 + j;
-                if (r < n && c < n) C[r * ld + c] = acc[i][j];
-            }
-    }
-    __syncthreads();
+    if constexpr (RIGHT_REAL)
+        prod_mma<CT, RT, RND, PROD_REAL_R, SH>(n, ld, C, op_n(static_cast<const cplx*>(Ap), ld), MatOp{},
+                                               static_cast<const double*>(Bp), TRI_NONE);
+    else
+        prod_mma<RT, CT, RND, PROD_REAL_L, SH>(n, ld, C, MatOp{}, op_n(static_cast<const cplx*>(Bp), ld),
+                                               static_cast<const double*>(Ap), TRI_NONE);
 }
 
 // dst = op(src) elementwise copy for an n x n matrix (dst must not alias src

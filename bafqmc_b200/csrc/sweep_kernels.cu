@@ -18,6 +18,8 @@ namespace bq {
 __constant__ uint32_t c_apow[kMaxPow];   // a^k mod 2^31 for k = 0 .. kMaxPow-1
 
 template <int NMAX> struct Cfg;
+// MR x MC tiles of 8 x 8 real elements per group and MQ groups per warp for the
+// products (mma64.cuh).
 // R8 rows per lane and CPS columns per 8-lane segment for the register-resident
 // factorisation routines: R8 >= NMAX/8, CPS >= NMAX/(THREADS/8).
 // LD: leading dimension of the shared-memory matrices, odd so that a column
@@ -29,6 +31,7 @@ template <> struct Cfg<16> {
     static constexpr int THREADS = 128, TR = 1, TC = 2, MAXE = 2, KB = 4, R8 = 2, CPS = 1, LD = 17, MINB = 2;
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 1, CPW = 1;
+    static constexpr int MR = 1, MC = 2, MQ = 1;
 };
 static_assert(16 % 1 == 0 && 16 % 2 == 0, "tile must divide NMAX");
 // N <= 36: two CTAs per SM, all four matrices in shared memory.  (Three CTAs
@@ -39,6 +42,7 @@ template <> struct Cfg<36> {
     static constexpr int THREADS = 256, TR = 2, TC = 3, MAXE = 6, KB = 4, R8 = 5, CPS = 2, LD = 37, MINB = 2;
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 2, CPW = 1;
+    static constexpr int MR = 1, MC = 3, MQ = 2;
 };
 // N <= 72: G and U in shared memory, the workspaces in HBM (one CTA per SM)
 template <> struct Cfg<72> {
@@ -46,6 +50,7 @@ template <> struct Cfg<72> {
     static constexpr int THREADS = 512, TR = 3, TC = 4, MAXE = 11, KB = 4, R8 = 9, CPS = 2, LD = 73, MINB = 1;
     static constexpr bool GW = true, GG = false;
     static constexpr int RW = 3, CPW = 1;
+    static constexpr int MR = 2, MC = 3, MQ = 2;
 };
 // N <= 144 (up to the 12x12 lattice, number-conserving): G, U, both
 // workspaces and a product scratch in HBM after the chain's arena (L2-resident
@@ -62,11 +67,17 @@ template <> struct Cfg<144> {
     static constexpr int RW = 5, CPW = 2;
 };
 template <int NMAX>
+constexpr bool mma_fits() {   // MQ rounds of the CTA's warps cover every group of tiles
+    using C = Cfg<NMAX>;
+    if constexpr (C::GG) return true;
+    else return C::MQ * (C::THREADS / 32) >= (((NMAX + 7) / 8 + C::MR - 1) / C::MR) * (((NMAX + 3) / 4 + C::MC - 1) / C::MC);
+}
+template <int NMAX>
 constexpr bool cfg_ok() {
     using C = Cfg<NMAX>;
     return NMAX % C::TR == 0 && NMAX % C::TC == 0 && (C::GG || (NMAX / C::TR) * (NMAX / C::TC) <= C::THREADS) &&
            (!C::GG || (C::RW * 32 >= NMAX && C::THREADS >= NMAX && C::GW)) &&
-           C::MAXE * C::THREADS >= NMAX * NMAX && C::R8 * 8 >= NMAX && C::CPS * (C::THREADS / 8) >= NMAX &&
+           mma_fits<NMAX>() && C::MAXE * C::THREADS >= NMAX * NMAX && C::R8 * 8 >= NMAX && C::CPS * (C::THREADS / 8) >= NMAX &&
            (C::LD & 1) == 1 && C::LD >= NMAX;
 }
 static_assert(cfg_ok<16>() && cfg_ok<36>() && cfg_ok<72>() && cfg_ok<144>(),
@@ -209,7 +220,7 @@ DEVI void gemm_any(Ctx<NMAX>& x, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) 
         gemm_big<C_::TR, C_::TC>(x.n, C_::LD, x.S(), A, B, tri);
         copy_mat(x.n, C_::LD, C, x.S());
     } else {
-        gemm_rs<C_::TR, C_::TC>(x.n, C_::LD, C, A, B, tri);
+        gemm_rs<C_::MR, C_::MC, C_::MQ, !C_::GW>(x.n, C_::LD, C, A, B, tri);
     }
 }
 template <int NMAX, bool RIGHT_REAL>
@@ -219,7 +230,7 @@ DEVI void gemm_real_any(Ctx<NMAX>& x, cplx* C, const void* A, const void* B) {
         gemm_big_real<C_::TR, C_::TC, RIGHT_REAL>(x.n, C_::LD, x.S(), A, B);
         copy_mat(x.n, C_::LD, C, x.S());
     } else {
-        gemm_smem_real<C_::TR, C_::TC, RIGHT_REAL>(x.n, C_::LD, C, A, B);
+        gemm_smem_real<C_::MR, C_::MC, C_::MQ, RIGHT_REAL, !C_::GW>(x.n, C_::LD, C, A, B);
     }
 }
 template <int NMAX>
