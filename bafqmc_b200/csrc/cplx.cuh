@@ -43,6 +43,17 @@ DEVI cplx cdiv(cplx a, cplx b) {
         return cmk((a.x * r + a.y) / den, (a.y * r - a.x) / den);
     }
 }
+// 1 / x for the serial chains: the approximate reciprocal (measured within 1e-6) and
+// one cubically convergent step of the Newton family, y (1 + e + e^2) with e = 1 - x y
+// (within 1.01 ulp of 1.0 / x over 2^-100 .. 2^100, measured).  No branch: the
+// compiler's division ends a basic block, and nothing is scheduled across it.
+// x = 0 and infinite x give NaN.
+DEVI double rcp_fast(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
 // exp(z) for complex z
 DEVI cplx cexpz(cplx z) {
     double s, c;
@@ -50,6 +61,19 @@ DEVI cplx cexpz(cplx z) {
     double e = exp(z.x);
     return cmk(e * c, e * s);
 }
+
+// A value that every lane of the warp holds, in a form the compiler takes as uniform.
+// Shuffles and mma under a branch or in a loop whose condition it cannot prove uniform
+// (a value from memory, threadIdx.x >> 5, a call's argument) are each preceded by a
+// warp synchronisation.
+DEVI int uni(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+DEVI int warp_index() { return uni((int)threadIdx.x >> 5); }
+
+// e / n by one multiplication, for loops over matrix elements (an integer division by a
+// runtime n costs about 40 instructions): q = umulhi(e, m), m = floor((2^32 - 1) / n) + 1,
+// exact for e n < 2^32 and n > 1 (and for e = 0).
+DEVI uint32_t div_magic(int n) { return 0xffffffffu / (uint32_t)n + 1u; }
+DEVI int div_by(int e, uint32_t m) { return (int)__umulhi((uint32_t)e, m); }
 
 DEVI double warp_sum(double v) {
 #pragma unroll

@@ -21,29 +21,26 @@
 
 // C = A * B for n x n operands (C may alias A or B), the complex product of
 // prod_mma out of line.  tri as there.
-template <int RT, int CT, int RND, bool SH>
+template <int RND, int NB, bool SH>
 COLD void gemm_rs(int n, int ld, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) {
-    prod_mma<RT, CT, RND, PROD_CC, SH>(n, ld, C, A, B, nullptr, tri);
+    prod_mma<RND, NB, PROD_CC, SH>(n, ld, C, A, B, nullptr, 0, tri);
 }
 
 // The slice propagators e^{-+dtau K} are real (real hopping, chemical
-// potential and pairing amplitude), so the per-slice products are complex x
-// real.  Real operands are stored as doubles with the same leading dimension.
-template <int RT, int CT, int RND, bool RIGHT_REAL, bool SH>
-DEVI void gemm_smem_real(int n, int ld, cplx* C, const void* Ap, const void* Bp) {
-    if constexpr (RIGHT_REAL)
-        prod_mma<CT, RT, RND, PROD_REAL_R, SH>(n, ld, C, op_n(static_cast<const cplx*>(Ap), ld), MatOp{},
-                                               static_cast<const double*>(Bp), TRI_NONE);
-    else
-        prod_mma<RT, CT, RND, PROD_REAL_L, SH>(n, ld, C, MatOp{}, op_n(static_cast<const cplx*>(Bp), ld),
-                                               static_cast<const double*>(Ap), TRI_NONE);
+// potential and pairing amplitude), so the per-slice products X <- X R or R X (and
+// X2 alike) are complex x real.  Real operands are stored as doubles with leading
+// dimension ldr (real_ld of the class).
+template <int RND, int NB, bool RIGHT_REAL, bool SH>
+COLD void gemm_smem_real(int n, int ld, int ldr, cplx* X, const double* R, cplx* X2 = nullptr) {
+    prod_mma<RND, NB, RIGHT_REAL ? PROD_REAL_R : PROD_REAL_L, SH>(n, ld, X, MatOp{}, MatOp{}, R, ldr, TRI_NONE, X2);
 }
 
 // dst = op(src) elementwise copy for an n x n matrix (dst must not alias src
 // unless op is the identity view).
 COLD void copy_op(int n, int ld, cplx* dst, MatOp src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * ld + c] = src.at(r, c);
     }
     __syncthreads();
@@ -52,12 +49,13 @@ COLD void copy_op(int n, int ld, cplx* dst, MatOp src) {
 // In-place conjugate transpose via register staging; MAXE >= ceil(n*n/blockDim).
 template <int MAXE>
 COLD void conj_transpose_inplace(int n, int ld, cplx* A) {
+    const uint32_t dm = div_magic(n);
     cplx v[MAXE];
 #pragma unroll
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e - (e / n) * n;
+            const int r = div_by(e, dm), c = e - r * n;
             v[k] = cconj(A[c * ld + r]);
         }
     }
@@ -66,7 +64,7 @@ COLD void conj_transpose_inplace(int n, int ld, cplx* A) {
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e - (e / n) * n;
+            const int r = div_by(e, dm), c = e - r * n;
             A[r * ld + c] = v[k];
         }
     }
@@ -152,6 +150,7 @@ struct QRScratch {
 // R8 >= ceil(n/8) rows per lane, CPS >= ceil(n/segments) columns per segment.
 template <int R8, int CPS>
 COLD void qrp_inplace(int n, int ld, cplx* A, QRScratch s) {
+    const uint32_t dm = div_magic(n);
     const int tid = threadIdx.x, lane = tid & 31, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
     const double tol3z = 1.0536712127723509e-08;   // sqrt(2^-53), LAPACK's sqrt(dlamch('E'))
     for (int j = seg; j < n; j += nseg) {
@@ -312,7 +311,7 @@ COLD void qrp_inplace(int n, int ld, cplx* A, QRScratch s) {
     }
     __syncthreads();
     for (int e = tid; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         if (c >= r) {
             const double x = s.vn1[r];
             const cplx a = A[r * ld + c];
@@ -582,12 +581,13 @@ COLD void trsm_right_upperH(int n, int ld, const cplx* F, const cplx* rinv, cons
 // i.e. P^T X); backward: out[piv[k]][:] = in[k][:] (ZLAPMR .false., i.e. P X).
 template <int MAXE>
 COLD void permute_rows(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward) {
+    const uint32_t dm = div_magic(n);
     cplx v[MAXE];
 #pragma unroll
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e % n;
+            const int r = div_by(e, dm), c = e - r * n;
             v[k] = C[(forward ? piv[r] : ipiv[r]) * ld + c];
         }
     }
@@ -596,7 +596,7 @@ COLD void permute_rows(int n, int ld, cplx* C, const int* piv, const int* ipiv, 
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e - (e / n) * n;
+            const int r = div_by(e, dm), c = e - r * n;
             C[r * ld + c] = v[k];
         }
     }
@@ -607,12 +607,13 @@ COLD void permute_rows(int n, int ld, cplx* C, const int* piv, const int* ipiv, 
 // .true., X P); backward: out[:, piv[k]] = in[:, k] (ZLAPMT .false., X P^T).
 template <int MAXE>
 COLD void permute_cols(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward) {
+    const uint32_t dm = div_magic(n);
     cplx v[MAXE];
 #pragma unroll
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e % n;
+            const int r = div_by(e, dm), c = e - r * n;
             v[k] = C[r * ld + (forward ? piv[c] : ipiv[c])];
         }
     }
@@ -621,7 +622,7 @@ COLD void permute_cols(int n, int ld, cplx* C, const int* piv, const int* ipiv, 
     for (int k = 0; k < MAXE; ++k) {
         const int e = threadIdx.x + k * blockDim.x;
         if (e < n * n) {
-            const int r = e / n, c = e - (e / n) * n;
+            const int r = div_by(e, dm), c = e - r * n;
             C[r * ld + c] = v[k];
         }
     }

@@ -205,8 +205,9 @@ COLD void gemm_big_real(int n, int ld, cplx* C, const void* Ap, const void* Bp) 
 }
 
 COLD void copy_mat(int n, int ld, cplx* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * ld + c] = src[r * ld + c];
     }
     __syncthreads();
@@ -220,16 +221,18 @@ COLD void conj_transpose_big(int n, int ld, cplx* A, cplx* S) {
 
 // Row / column permutations as permute_rows / permute_cols, through S.
 COLD void permute_rows_big(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward, cplx* S) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         S[r * ld + c] = C[(forward ? piv[r] : ipiv[r]) * ld + c];
     }
     __syncthreads();
     copy_mat(n, ld, C, S);
 }
 COLD void permute_cols_big(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward, cplx* S) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         S[r * ld + c] = C[r * ld + (forward ? piv[c] : ipiv[c])];
     }
     __syncthreads();
@@ -395,8 +398,9 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
         s.vn1[i] = 1.0 / d;
     }
     __syncthreads();
+    const uint32_t dm = div_magic(n);
     for (int e = tid; e < n * n; e += blockDim.x) {
-        const int q = e / n, t = e - q * n;   // consecutive threads walk the storage order
+        const int q = div_by(e, dm), t = e - q * n;   // consecutive threads walk the storage order
         const int r = CM ? t : q, c = CM ? q : t;
         if (c >= r) {
             const double x = s.vn1[r];
@@ -414,8 +418,9 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
 // reflector and triangular-solve routines below read F one column per warp;
 // with FCM they read such a copy, so each warp load is one contiguous segment.
 COLD void copy_col_major(int n, int ld, cplx* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - r * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[c * ld + r] = src[r * ld + c];
     }
     __syncthreads();

@@ -18,8 +18,8 @@ namespace bq {
 __constant__ uint32_t c_apow[kMaxPow];   // a^k mod 2^31 for k = 0 .. kMaxPow-1
 
 template <int NMAX> struct Cfg;
-// MR x MC tiles of 8 x 8 real elements per group and MQ groups per warp for the
-// products (mma64.cuh).
+// MQ tiles per warp, MB at a time, for the complex products and MP for the real ones
+// (mma64.cuh).
 // R8 rows per lane and CPS columns per 8-lane segment for the register-resident
 // factorisation routines: R8 >= NMAX/8, CPS >= NMAX/(THREADS/8).
 // LD: leading dimension of the shared-memory matrices, odd so that a column
@@ -28,10 +28,10 @@ template <int NMAX> struct Cfg;
 // only G and U in shared memory.
 template <> struct Cfg<16> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 128, TR = 1, TC = 2, MAXE = 2, KB = 4, R8 = 2, CPS = 1, LD = 17, MINB = 2;
+    static constexpr int THREADS = 128, TR = 1, TC = 2, MAXE = 2, KB = 8, R8 = 2, CPS = 1, LD = 17, MINB = 4;
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 1, CPW = 1;
-    static constexpr int MR = 1, MC = 2, MQ = 1;
+    static constexpr int LEADS = 1, MQ = 1, MB = 1, MP = 2;
 };
 static_assert(16 % 1 == 0 && 16 % 2 == 0, "tile must divide NMAX");
 // N <= 36: two CTAs per SM, all four matrices in shared memory.  (Three CTAs
@@ -39,18 +39,18 @@ static_assert(16 % 1 == 0 && 16 % 2 == 0, "tile must divide NMAX");
 // slice products and wraps slow down more than the third chain adds.)
 template <> struct Cfg<36> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 256, TR = 2, TC = 3, MAXE = 6, KB = 4, R8 = 5, CPS = 2, LD = 37, MINB = 2;
+    static constexpr int THREADS = 256, TR = 2, TC = 3, MAXE = 6, KB = 8, R8 = 5, CPS = 2, LD = 37, MINB = 2;
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 2, CPW = 1;
-    static constexpr int MR = 1, MC = 3, MQ = 2;
+    static constexpr int LEADS = 2, MQ = 4, MB = 2, MP = 8;
 };
 // N <= 72: G and U in shared memory, the workspaces in HBM (one CTA per SM)
 template <> struct Cfg<72> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 512, TR = 3, TC = 4, MAXE = 11, KB = 4, R8 = 9, CPS = 2, LD = 73, MINB = 1;
+    static constexpr int THREADS = 512, TR = 3, TC = 4, MAXE = 11, KB = 8, R8 = 9, CPS = 2, LD = 73, MINB = 1;
     static constexpr bool GW = true, GG = false;
     static constexpr int RW = 3, CPW = 1;
-    static constexpr int MR = 2, MC = 3, MQ = 2;
+    static constexpr int LEADS = 1, MQ = 6, MB = 2, MP = 6;
 };
 // N <= 144 (up to the 12x12 lattice, number-conserving): G, U, both
 // workspaces and a product scratch in HBM after the chain's arena (L2-resident
@@ -61,16 +61,17 @@ template <> struct Cfg<72> {
 static_assert(kTcPer * 512 >= 144 * kTcKC, "tensor-core staging: elements per thread must cover a chunk");
 template <> struct Cfg<144> {
     static constexpr bool TCORE = true;   // slice products may run on the tensor cores (tc.cuh)
-    static constexpr int THREADS = 512, TR = 2, TC = 3, MAXE = 41, KB = 4, R8 = 18, CPS = 3, LD = 145,
+    static constexpr int THREADS = 512, TR = 2, TC = 3, MAXE = 41, KB = 8, R8 = 18, CPS = 3, LD = 145,
                          MINB = 1;
     static constexpr bool GW = true, GG = true;
+    static constexpr int LEADS = 1;
     static constexpr int RW = 5, CPW = 2;
 };
 template <int NMAX>
-constexpr bool mma_fits() {   // MQ rounds of the CTA's warps cover every group of tiles
+constexpr bool mma_fits() {   // the CTA's warps hold every tile of a product
     using C = Cfg<NMAX>;
     if constexpr (C::GG) return true;
-    else return C::MQ * (C::THREADS / 32) >= (((NMAX + 7) / 8 + C::MR - 1) / C::MR) * (((NMAX + 3) / 4 + C::MC - 1) / C::MC);
+    else return C::MQ * (C::THREADS / 32) >= mma_tiles(NMAX) && C::MP * (C::THREADS / 32) >= mma_tiles(NMAX);
 }
 template <int NMAX>
 constexpr bool cfg_ok() {
@@ -98,10 +99,14 @@ struct Smem {
     static constexpr bool GG = Cfg<NMAX>::GG;   // G and U in HBM as well
     static constexpr size_t oG = 0, oU = MM, oW1 = 2 * MM, oW2 = 3 * MM;
     static constexpr int KB = Cfg<NMAX>::KB;
-    static constexpr size_t oTau = (GG ? 0 : (GW ? 2 : 4)) * MM, oCol = oTau + VC, oRow = oCol + KB * VC, oDelta = oRow + KB * VC;
+    // block vectors X and Y, at an odd stride: the mma fragments over slots and rows fall in distinct banks (mma64.cuh)
+    static constexpr int VS = NMAX + 1;
+    static constexpr size_t BV = sizeof(cplx) * VS * KB, BB = sizeof(cplx) * KB * KB;
+    static constexpr size_t oTau = (GG ? 0 : (GW ? 2 : 4)) * MM, oCol = oTau + VC, oRow = oCol + BV;
+    static constexpr size_t oXb = oRow + BV, oYb = oXb + BB, oSnap = oYb + BB, oFld = oSnap + BB, oDelta = oFld + VC;
     static constexpr size_t oDelta2 = oDelta + VC;
     static constexpr size_t oEao = oDelta2 + VC, oEan = oEao + VC, oEbo = oEan + VC, oEbn = oEbo + VC;
-    static constexpr size_t oPh = oEbn + VC, oCoef = oPh + VC, oCbc = oCoef + KB * sizeof(cplx);
+    static constexpr size_t oPh = oEbn + VC, oCoef = oPh + VC, oCbc = oCoef + 2 * KB * sizeof(cplx);
     static constexpr size_t oP = oCbc + 4 * sizeof(cplx);
     static constexpr size_t oRg = oP + ((sizeof(PointDev) + 15) / 16) * 16;
     static constexpr size_t oU2 = oRg + VD, oPhin = oU2 + VD, oVn1 = oPhin + VD, oVn2 = oVn1 + VD, oD = oVn2 + VD;
@@ -125,8 +130,12 @@ struct Smem {
     DEVI cplx* W1() const { return at<cplx>(oW1); }   // shared-memory workspaces (N <= 36 classes)
     DEVI cplx* W2() const { return at<cplx>(oW2); }
     DEVI cplx* tau() const { return at<cplx>(oTau); }
-    DEVI cplx* col(int m) const { return at<cplx>(oCol) + m * NMAX; }   // column of the m-th site of a block
-    DEVI cplx* row(int m) const { return at<cplx>(oRow) + m * NMAX; }   // row of the m-th site of a block
+    DEVI cplx* col(int m) const { return at<cplx>(oCol) + m * VS; }   // X of slot m of a block
+    DEVI cplx* row(int m) const { return at<cplx>(oRow) + m * VS; }   // Y of slot m
+    DEVI cplx* xb() const { return at<cplx>(oXb); }   // X and Y of a block on its own slots, [m][slot]
+    DEVI cplx* yb() const { return at<cplx>(oYb); }
+    DEVI double* fld() const { return at<double>(oFld); }   // fields of the slice under update, [site][channel]
+    DEVI cplx* snap() const { return at<cplx>(oSnap); }   // submatrix of G at the start of the next block
     DEVI cplx* delta() const { return at<cplx>(oDelta); }
     DEVI cplx* delta2() const { return at<cplx>(oDelta2); }   // Nambu: Delta of the c^dagger index
     DEVI cplx* eao() const { return at<cplx>(oEao); }
@@ -209,6 +218,9 @@ struct Ctx {
     DEVI cplx* S() const { return wg + 4 * NMAX * Cfg<NMAX>::LD; }   // product scratch (HBM-resident classes)
 };
 
+// leading dimension of a class's real e^{-+dtau K}
+template <int NMAX> constexpr int kLdReal = Cfg<NMAX>::GG ? Cfg<NMAX>::LD : real_ld(NMAX);
+
 // ---------------------------------------------------------------------------
 // Linear algebra per size class: the register-resident 8-lane-segment
 // routines of linalg.cuh for the shared-memory classes, the warp-per-column
@@ -220,17 +232,23 @@ DEVI void gemm_any(Ctx<NMAX>& x, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) 
         gemm_big<C_::TR, C_::TC>(x.n, C_::LD, x.S(), A, B, tri);
         copy_mat(x.n, C_::LD, C, x.S());
     } else {
-        gemm_rs<C_::MR, C_::MC, C_::MQ, !C_::GW>(x.n, C_::LD, C, A, B, tri);
+        gemm_rs<C_::MQ, C_::MB, !C_::GW>(x.n, C_::LD, C, A, B, tri);
     }
 }
+// X <- X R (RIGHT_REAL) or R X, and X2 alike if given (classes with operands in shared memory)
 template <int NMAX, bool RIGHT_REAL>
-DEVI void gemm_real_any(Ctx<NMAX>& x, cplx* C, const void* A, const void* B) {
+DEVI void gemm_real_any(Ctx<NMAX>& x, cplx* X, const double* R, cplx* X2 = nullptr) {
     using C_ = Cfg<NMAX>;
     if constexpr (C_::GG) {
-        gemm_big_real<C_::TR, C_::TC, RIGHT_REAL>(x.n, C_::LD, x.S(), A, B);
-        copy_mat(x.n, C_::LD, C, x.S());
+        if (RIGHT_REAL) gemm_big_real<C_::TR, C_::TC, true>(x.n, C_::LD, x.S(), X, R);
+        else gemm_big_real<C_::TR, C_::TC, false>(x.n, C_::LD, x.S(), R, X);
+        copy_mat(x.n, C_::LD, X, x.S());
+        if (X2) gemm_real_any<NMAX, RIGHT_REAL>(x, X2, R);
     } else {
-        gemm_smem_real<C_::MR, C_::MC, C_::MQ, RIGHT_REAL, !C_::GW>(x.n, C_::LD, C, A, B);
+        // both in one call if the CTA's warps hold both results (they wait in registers)
+        const bool two = X2 && 2 * mma_tiles(x.n) > C_::MP * (C_::THREADS / 32);
+        gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, kLdReal<NMAX>, X, R, two ? nullptr : X2);
+        if (two) gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, kLdReal<NMAX>, X2, R, nullptr);
     }
 }
 template <int NMAX>
@@ -240,15 +258,16 @@ DEVI void qrp_any(Ctx<NMAX>& x, cplx* A) {
         // factorised in a column-major copy in S, so each warp's column walk is
         // contiguous; the operations and their order are those of the row-major call
         const int n = x.n;
+    const uint32_t dm = div_magic(n);
         cplx* S = x.S();
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-            const int r = e / n, c = e - r * n;
+            const int r = div_by(e, dm), c = e - r * n;
             S[c * C_::LD + r] = A[r * C_::LD + c];
         }
         __syncthreads();
         qrp_big<C_::RW, true>(n, C_::LD, S, x.s.qr());
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-            const int r = e / n, c = e - r * n;
+            const int r = div_by(e, dm), c = e - r * n;
             A[r * C_::LD + c] = S[c * C_::LD + r];
         }
         __syncthreads();
@@ -335,8 +354,7 @@ DEVI void slice_mult(Ctx<NMAX>& x, cplx* X, const double* R) {
             __syncthreads();
         }
     }
-    if constexpr (RIGHT) gemm_real_any<NMAX, true>(x, X, X, R);
-    else gemm_real_any<NMAX, false>(x, X, R, X);
+    gemm_real_any<NMAX, RIGHT>(x, X, R);
 }
 
 // Tensor memory and the MMA barrier of a CTA that runs mixed-precision products
@@ -387,27 +405,31 @@ DEVI void gcopy(cplx* dst, const cplx* src, int count) {
 }
 // identity in an n x n matrix with leading dimension ld
 DEVI void set_identity(int n, int ld, cplx* A) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         A[r * ld + c] = cmk(r == c ? 1.0 : 0.0, 0.0);
     }
 }
 // dense n x n (global) <-> shared n x n with leading dimension ld
 DEVI void sload(int n, int ld, cplx* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * ld + c] = src[e];
     }
 }
 DEVI void sstore(int n, int ld, cplx* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[e] = src[r * ld + c];
     }
 }
 DEVI void scopy(int n, int ld, cplx* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * ld + c] = src[r * ld + c];
     }
 }
@@ -415,15 +437,16 @@ DEVI void scopy(int n, int ld, cplx* dst, const cplx* src) {
 // e^{-dtau K} (real) into W1 and e^{+dtau K} into W2 as doubles with the
 // matrices' leading dimension.
 DEVI void sload_real(int n, int ld, double* dst, const cplx* src) {
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * ld + c] = src[e].x;
     }
 }
 template <int NMAX>
 DEVI void load_expT(Ctx<NMAX>& x) {
-    sload_real(x.n, Cfg<NMAX>::LD, reinterpret_cast<double*>(x.W1()), x.P().expP);
-    sload_real(x.n, Cfg<NMAX>::LD, reinterpret_cast<double*>(x.W2()), x.P().expM);
+    sload_real(x.n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
+    sload_real(x.n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W2()), x.P().expM);
     __syncthreads();
 }
 
@@ -432,15 +455,8 @@ DEVI void load_expT(Ctx<NMAX>& x) {
 // V-wrap of G (LocalU_prop_L / LocalU_prop_R, localU.f90:79-113, and
 // LocalU_metro, localU.f90:31-77).
 //
-// Sites are strictly sequential.  They are taken in blocks of KB consecutive
-// sites.  Within a block one warp runs the sites one after another, with
-// warp-level synchronisation only: for each site it wraps and records the
-// site's column and row, makes the Metropolis decision (every lane computes
-// the same one), and applies the rank-1 update to the rows and columns of the
-// block's sites -- the only elements the block's later sites read.  After the
-// block, the whole CTA adds the block's KB rank-1 terms to the remaining
-// elements, which the wraps of the block's sites do not touch.  The terms are
-// the reference's ZGERU updates; only the order of the additions changes.
+// Sites are strictly sequential.  The terms are the reference's updates; only the
+// order of the additions changes.
 
 // e^{+alpha phi} and e^{-alpha phi} for the HS coupling alpha = ar + i ai of one
 // channel, which the reference makes purely real (U2) or purely imaginary (U1)
@@ -467,73 +483,81 @@ DEVI cplx ratio_unit(double ar, double ai, cplx en, cplx eo) {
     return cdiv(en, eo);
 }
 
-// Metropolis ratio for the (wrapped) diagonal element gjj: ratio_det = 1/w,
-// w = 1 + Delta (1 - G_jj); accept if r_gauss |ratio_det|^2 > u; on accept the
-// rank-1 coefficient is -ratio_det * Delta (localU.f90:56-71).
-DEVI bool metro_ratio(cplx d, double rg, double u, cplx gjj, cplx& coef) {
-    const cplx w = cmk(1.0 + (d.x * (1.0 - gjj.x) + d.y * gjj.y), d.y * (1.0 - gjj.x) - d.x * gjj.y);
-    const double inv = 1.0 / (w.x * w.x + w.y * w.y);
-    const bool accept = rg * inv > u;
-    const cplx t = cmulcj(d, w);   // Delta * conj(w)
-    coef = accept ? cmk(-t.x * inv, -t.y * inv) : cmk(0.0, 0.0);
-    return accept;
-}
-
-// prop_channel visits the sites of a channel in blocks of KB.  Per block:
+// prop_channel visits the sites of a channel in blocks of KB slots, one slot per
+// site of a number-conserving chain and two (b_i, c^dagger_i) per site of a
+// Nambu chain.  Per block:
 //  1. lead_block: one warp makes the block's Metropolis decisions in visiting
 //     order on the block's kb x kb submatrix of G, held in registers, applying
-//     each accepted rank-1 term to the submatrix (no barrier per site);
+//     each accepted term to the submatrix (no barrier per site);
 //  2. block_vectors: the full update vectors of the block from the recorded
 //     coefficients and block values;
-//  3. rank_tile / rank_rows: G += sum_m X_m Y_m^T on every element.
-// The rank-1 term of a site i (localU.f90:56-71, ZGERU) is
-// G <- G + coef G(:,i) (e_i - G(i,:))^T.  For any diagonal E it satisfies
-// F_i(E G E^-1) = E F_i(G) E^-1, and coef depends only on G(i,i), which E
-// leaves unchanged, so the wraps of the sites (row i by e^{a phi_i}, column i
-// by e^{-a phi_i} before the decision in the right traversal, with the old
-// field; row i by e^{-a phi_i} and column i by e^{a phi_i} after it in the left
-// traversal, with the final field) commute with the updates and are applied
-// once, as one diagonal similarity, in the last block's rank pass.
+//  3. rank_tiles / rank_rows: G += sum_m X_m Y_m^T on every element.
+// Number-conserving (localU.f90:56-71, ZGERU): the rank-1 term of site i is
+// G <- G + coef G(:,i) (e_i - G(i,:))^T.  Nambu (src/pairing/src/localU.f90:33-149
+// on the {b, c^dagger} block): the reference forms the 4x4 P = I + Delta (I -
+// G[isec,isec]) over the sectors of the site, takes ratio_det = det(P)^(-1/2), and
+// on acceptance G -= G[:,isec] P^{-1} Delta (I[isec,:] - G[isec,:]).  P splits into
+// the 2x2 block P1 on s = (i, Ns+i) and its complex conjugate, so det(P) = |det P1|^2
+// (real and positive: the phase that PhaseCounter records is zero), and the block's
+// term is the rank-2 G1 -= G1[:,s] P1^{-1} D1 (I[s,:] - G1[s,:]).
+// For any diagonal E both satisfy F_i(E G E^-1) = E F_i(G) E^-1, and the ratio is
+// that of G (a Nambu P1 becomes E P1 E^-1), so the wraps of the sites (row i by
+// e^{a phi_i}, column i by e^{-a phi_i} before the decision in the right traversal,
+// with the old field; row i by e^{-a phi_i} and column i by e^{a phi_i} after it in
+// the left traversal, with the final field) commute with the updates and are
+// applied once, as one diagonal similarity, in the last block's rank pass.
+//
+// Eight slots a block: what a block costs besides its decisions (two barriers, the
+// vectors, the pass's loads and stores of G) is paid per eight slots, and the
+// decisions (a chain of shuffle, ratio, reciprocal and update per site) run beside
+// the pass, which takes the FP64 tensor pipe.  Bound: the decisions (about 300 cycles
+// a site on their own) and the vectors (1.3 K cycles a block).  Against blocks of four
+// with a DFMA pass (number-conserving) and one barrier per site with every thread
+// keeping its elements (Nambu), M cycles of updates per sweep of a chain: 6x6 Nambu
+// block, L = 40, one CTA per SM 89 -> 13.7; 4x4 Nambu, two CTAs 12.8 -> 5.9; 8x8,
+// L = 40 24.0 -> 9.7; 12x12, L = 50 181 -> 144; 6x6, L = 160, two CTAs 26.2 -> 26.4.
+static_assert(Cfg<16>::KB == 8 && Cfg<36>::KB == 8 && Cfg<72>::KB == 8 && Cfg<144>::KB == 8,
+              "the lead warp holds the block's 8 x 8 submatrix, two rows per lane");
 
-static_assert(Cfg<16>::KB * Cfg<16>::KB <= 16 && Cfg<36>::KB * Cfg<36>::KB <= 16 && Cfg<72>::KB * Cfg<72>::KB <= 16 &&
-                  Cfg<144>::KB * Cfg<144>::KB <= 16,
-              "the block records (tau, delta2, the vn1 | vn2 snapshot) hold KB x KB values in NMAX >= 16 entries, "
-              "and the lead warp one element per lane");
+// matrix index of slot k of the block that starts at the k0-th visited site
+template <bool LEFT, bool PAIR>
+DEVI int slot_index(int ns, int k0, int k) {
+    const int m = k0 + (PAIR ? k >> 1 : k);
+    return (LEFT ? ns - 1 - m : m) + (PAIR && (k & 1) ? ns : 0);
+}
 
 // the channel's deferred wrap: factor of row r and of column c
-template <int NMAX, bool LEFT>
-DEVI cplx wrap_row(const Smem<NMAX>& s, int r) {
-    if constexpr (LEFT) return s.accf()[r] ? s.ebn()[r] : s.ebo()[r];
-    else return s.eao()[r];
+template <int NMAX, bool LEFT, bool PAIR>
+DEVI cplx wrap_row(const Ctx<NMAX>& x, int r, bool flip) {
+    const auto& s = x.s;
+    const bool cd = PAIR && r >= x.P().Ns;
+    const int i = cd ? r - x.P().Ns : r;
+    const bool up = (cd && flip) != !LEFT;   // e^{+alpha phi} rather than e^{-alpha phi}
+    if constexpr (LEFT) return s.accf()[i] ? (up ? s.ean()[i] : s.ebn()[i]) : (up ? s.eao()[i] : s.ebo()[i]);
+    else return up ? s.eao()[i] : s.ebo()[i];
 }
-template <int NMAX, bool LEFT>
-DEVI cplx wrap_col(const Smem<NMAX>& s, int c) {
-    if constexpr (LEFT) return s.accf()[c] ? s.ean()[c] : s.eao()[c];
-    else return s.ebo()[c];
+template <int NMAX, bool LEFT, bool PAIR>
+DEVI cplx wrap_col(const Ctx<NMAX>& x, int c, bool flip) {
+    const auto& s = x.s;
+    const bool cd = PAIR && c >= x.P().Ns;
+    const int i = cd ? c - x.P().Ns : c;
+    const bool up = (cd && flip) != LEFT;
+    if constexpr (LEFT) return s.accf()[i] ? (up ? s.ean()[i] : s.ebn()[i]) : (up ? s.eao()[i] : s.ebo()[i]);
+    else return up ? s.eao()[i] : s.ebo()[i];
 }
 
-// Step 1, by the lead warp (warp sw0 of the CTA).  Lane l < KB*KB holds
-// the element (l / KB, l % KB) of the block's kb x kb submatrix of the current
-// G; the decisions run in visiting order, every lane computing the same
-// Metropolis ratio from the diagonal element it receives by shuffle.  Records
-// per visited slot m: coef (coef()), X_m on the later block sites (xb = tau(),
-// [m][a], a > m) and Y_m on them (yb = delta2(), [m][b], b > m), where
-// X_m = coef G_{m-1}(:, i_m) and Y_m = e_{i_m} - G_{m-1}(i_m, :)^T.  Only the
-// trailing submatrix (sites after m) is updated: nothing later reads the
-// rest.  A rejected site has coef = 0, so its update adds exact zeros.
-
-// the submatrix at block start k0 into the QR norm vectors (vn1 | vn2, free
-// during local updates); the lead warp reads it back after the barrier, when
-// the rank pass may already be writing G
-template <int NMAX, bool LEFT>
-DEVI void block_snapshot(const Smem<NMAX>& s, const cplx* G, int n, int k0, int kb) {
+// the submatrix at block start k0 into snap(); the lead warp reads it back after
+// the barrier, when the rank pass may already be writing G
+template <int NMAX, bool LEFT, bool PAIR>
+DEVI void block_snapshot(const Ctx<NMAX>& x, const cplx* G, int k0, int kb) {
     constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD;
-    const int lane = threadIdx.x & 31;
-    if (lane < KB * KB) {
-        const int a = lane / KB, b = lane % KB;
-        const int sa = LEFT ? n - 1 - (k0 + min(a, kb - 1)) : k0 + min(a, kb - 1);
-        const int sb = LEFT ? n - 1 - (k0 + min(b, kb - 1)) : k0 + min(b, kb - 1);
-        reinterpret_cast<cplx*>(s.vn1())[lane] = (a < kb && b < kb) ? G[sa * LD + sb] : cmk(0.0, 0.0);
+    const int lane = threadIdx.x & 31, ns = x.P().Ns;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int a = (lane >> 3) + 4 * h, b = lane & 7;
+        cplx v = cmk(0.0, 0.0);
+        if (a < kb && b < kb) v = G[slot_index<LEFT, PAIR>(ns, k0, a) * LD + slot_index<LEFT, PAIR>(ns, k0, b)];
+        x.s.snap()[a * KB + b] = v;
     }
 }
 
@@ -541,132 +565,265 @@ DEVI cplx shfl_c(cplx v, int src) {
     return cmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// The snapshot, the previous block's kbp rank terms (in the order and with the
-// operations of the rank pass, so the lanes hold exactly the G the pass
-// writes there), then the decisions.  Returns the accepted count.
-template <int NMAX, bool LEFT>
-COLD long long lead_block(Ctx<NMAX> x, int n, int k0, int kb, int kbp) {
+// Step 1, by the lead warp (warp sw0 of the CTA).  Lane l holds the elements
+// (l / 8, l % 8) and (l / 8 + 4, l % 8) of the block's submatrix: the snapshot plus
+// the previous block's kbp terms (to rounding the G that the pass writes there).
+// The decisions run in visiting order, every lane computing the same ratio from the
+// elements it receives by shuffle.  Records per slot m: the coefficients (coef()),
+// X_m on the later block slots (xb, [m][a], a > m) and Y_m on them (yb, [m][b], b > m),
+// where X_m = coef G_{m-1}(:, i_m) and Y_m = e_{i_m} - G_{m-1}(i_m, :)^T (Nambu: the
+// two columns of -G[:,s] P1^{-1} D1 and the two rows of I[s,:] - G[s,:]).  Nothing
+// later reads the submatrix or the records at slots up to m, so every lane updates
+// and stores without a condition (lanes of one address hold one value): a divergent
+// branch costs about what the arithmetic of a site does.  A rejected site has zero coefficients, so its update adds exact zeros.  The accept
+// test r_g |ratio_det|^2 > u is taken as r_g > u |det|^2, which needs no division.
+// Returns the accepted count.
+template <int NMAX, bool LEFT, bool PAIR>
+COLD long long lead_block(Ctx<NMAX> x, int k0, int kb, int kbp) {
     constexpr int KB = Cfg<NMAX>::KB;
     const auto& s = x.s;
-    const int lane = threadIdx.x & 31;
-    const bool own = lane < KB * KB;
-    const int a = own ? lane / KB : KB - 1, b = lane % KB;
-    cplx* xb = s.tau();
-    cplx* yb = s.delta2();
-    cplx g = reinterpret_cast<const cplx*>(s.vn1())[a * KB + b];
-    if (kbp > 0 && a < kb && b < kb) {
-        const int sa = LEFT ? n - 1 - (k0 + a) : k0 + a, sb = LEFT ? n - 1 - (k0 + b) : k0 + b;
+    const int lane = threadIdx.x & 31, ns = uni(x.P().Ns);
+    const int b = lane & 7, a0 = lane >> 3;
+    k0 = uni(k0);
+    kb = uni(kb);
+    kbp = uni(kbp);
+    cplx *xb = s.xb(), *yb = s.yb();
+    cplx g[2];
+    const int ib = slot_index<LEFT, PAIR>(ns, k0, min(b, kb - 1));
 #pragma unroll
-        for (int m = 0; m < KB; ++m) {
-            if (m >= kbp) break;
-            g = cfma(s.col(m)[sa], s.row(m)[sb], g);
+    for (int h = 0; h < 2; ++h) {
+        const int a = a0 + 4 * h;
+        g[h] = s.snap()[a * KB + b];
+        const int ia = slot_index<LEFT, PAIR>(ns, k0, min(a, kb - 1));
+        if (kbp > 0) {   // all KB slots: block_vectors zeroes those that a short block does not have
+            cplx t = cmk(0.0, 0.0);   // two chains: slots 0..3 onto g, 4..7 onto t
+#pragma unroll
+            for (int m = 0; m < KB / 2; ++m) {
+                g[h] = cfma(s.col(m)[ia], s.row(m)[ib], g[h]);
+                t = cfma(s.col(m + KB / 2)[ia], s.row(m + KB / 2)[ib], t);
+            }
+            g[h] = cadd(g[h], t);
         }
     }
     long long nacc = 0;
+    if constexpr (!PAIR) {
+        int i = slot_index<LEFT, PAIR>(ns, k0, 0);
+        cplx d = s.delta()[i];
+        double rg = s.rg()[i], u = s.u2()[i];
 #pragma unroll
-    for (int m = 0; m < KB; ++m) {
-        if (m >= kb) break;
-        const int i = LEFT ? n - 1 - (k0 + m) : k0 + m;
-        const cplx gmm = shfl_c(g, m * KB + m);
-        const cplx gam = shfl_c(g, a * KB + m);
-        const cplx gmb = shfl_c(g, m * KB + b);
-        cplx coef;
-        const bool accept = metro_ratio(s.delta()[i], s.rg()[i], s.u2()[i], gmm, coef);
-        const cplx xv = cmul(coef, gam);
-        const cplx yv = cmk(-gmb.x, -gmb.y);
-        if (a > m && b > m) g = cfma(xv, yv, g);
-        if (own && b == m && a > m) xb[m * KB + a] = xv;
-        if (own && a == m && b > m) yb[m * KB + b] = yv;
-        if (lane == 0) {
+        for (int m = 0; m < KB; ++m) {
+            if (m >= kb) break;
+            const int src = (m & 3) << 3, hm = m >> 2;
+            const cplx gmm = shfl_c(g[hm], src | m);
+            const cplx gmb = shfl_c(g[hm], src | b);
+            cplx gam[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) gam[h] = shfl_c(g[h], (lane & 24) | m);
+            // w = 1 + Delta (1 - G_ii), coef = -Delta / w on acceptance (localU.f90:56-71)
+            const cplx w = cmk(1.0 + (d.x * (1.0 - gmm.x) + d.y * gmm.y), d.y * (1.0 - gmm.x) - d.x * gmm.y);
+            const double w2 = w.x * w.x + w.y * w.y;
+            const bool accept = rg > u * w2;
+            const double inv = rcp_fast(w2);
+            const cplx t = cmulcj(d, w);   // Delta * conj(w)
+            const cplx coef = cmk(accept ? -t.x * inv : 0.0, accept ? -t.y * inv : 0.0);
+            const int ni = slot_index<LEFT, PAIR>(ns, k0, min(m + 1, kb - 1));
+            d = s.delta()[ni];   // the next site's proposal, before this site's stores
+            rg = s.rg()[ni];
+            u = s.u2()[ni];
+            const cplx yv = cmk(-gmb.x, -gmb.y);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const cplx xv = cmul(coef, gam[h]);
+                g[h] = cfma(xv, yv, g[h]);
+                xb[m * KB + a0 + 4 * h] = xv;
+            }
+            yb[m * KB + b] = yv;
             s.accf()[i] = accept ? 1 : 0;
             s.coef()[m] = coef;
+            nacc += accept ? 1 : 0;
+            i = ni;
         }
-        nacc += accept ? 1 : 0;
+    } else {
+#pragma unroll 1
+        for (int m = 0; 2 * m < kb; ++m) {
+            const int i = slot_index<LEFT, PAIR>(ns, k0, 2 * m);
+            const cplx d0 = s.delta()[i], d1 = s.delta2()[i];
+            const double rg = s.rg()[i], u = s.u2()[i];
+            const int p = 2 * m, q = p + 1, sp = (p & 3) << 3, sq = (q & 3) << 3;
+            const cplx gm = p < 4 ? g[0] : g[1];
+            const cplx gaa = shfl_c(gm, sp | p), gab = shfl_c(gm, sp | q);
+            const cplx gba = shfl_c(gm, sq | p), gbb = shfl_c(gm, sq | q);
+            const cplx gpb = shfl_c(gm, sp | b), gqb = shfl_c(gm, sq | b);
+            cplx gap[2], gaq[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                gap[h] = shfl_c(g[h], (lane & 24) | p);
+                gaq[h] = shfl_c(g[h], (lane & 24) | q);
+            }
+            // P1 = I + D1 (I - G1[s,s]);  accept if |rg rc| > u |det P1|
+            const cplx p00 = cadd(cmk(1.0, 0.0), cmul(d0, cmk(1.0 - gaa.x, -gaa.y)));
+            const cplx p01 = cmul(d0, cmk(-gab.x, -gab.y));
+            const cplx p10 = cmul(d1, cmk(-gba.x, -gba.y));
+            const cplx p11 = cadd(cmk(1.0, 0.0), cmul(d1, cmk(1.0 - gbb.x, -gbb.y)));
+            const cplx det = csub(cmul(p00, p11), cmul(p01, p10));
+            const double det2 = det.x * det.x + det.y * det.y;
+            const bool accept = rg > u * sqrt(det2);
+            const double rr = rcp_fast(det2), inv = accept ? rr : 0.0;
+            // -M, M = P1^{-1} D1, P1^{-1} = adj(P1) conj(det) / |det|^2
+            const cplx id = cmk(-det.x * inv, det.y * inv);
+            const cplx e0 = cmul(id, d0), e1 = cmul(id, d1);
+            const cplx m00 = cmul(p11, e0), m01 = cmul(cmk(-p01.x, -p01.y), e1);
+            const cplx m10 = cmul(cmk(-p10.x, -p10.y), e0), m11 = cmul(p00, e1);
+            const cplx yp = cmk(-gpb.x, -gpb.y), yq = cmk(-gqb.x, -gqb.y);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int a = a0 + 4 * h;
+                const cplx xp = cfma(gaq[h], m10, cmul(gap[h], m00)), xq = cfma(gaq[h], m11, cmul(gap[h], m01));
+                g[h] = cfma(xq, yq, cfma(xp, yp, g[h]));
+                xb[p * KB + a] = xp;
+                xb[q * KB + a] = xq;
+            }
+            yb[p * KB + b] = yp;
+            yb[q * KB + b] = yq;
+            s.accf()[i] = accept ? 1 : 0;
+            s.coef()[4 * m] = m00;
+            s.coef()[4 * m + 1] = m01;
+            s.coef()[4 * m + 2] = m10;
+            s.coef()[4 * m + 3] = m11;
+            nacc += accept ? 1 : 0;
+        }
     }
     return nacc;
 }
 
-// Step 2.  X_k(r) = coef_k (G(r, i_k) + sum_{j<k} X_j(r) Y_j(i_k)) into col(k),
-// Y_k(c) = delta(c, i_k) - (G(i_k, c) + sum_{j<k} X_j(i_k) Y_j(c)) into row(k);
-// threads 0..n-1 build the X rows, n..2n-1 the Y columns.
-template <int NMAX, bool LEFT>
+// Step 2.  The update vectors on every row and column, from the block's starting G:
+// g_k(r) = G(r, i_k) + sum_{j<k} X_j(r) Y_j(i_k) gives X_k into col(k), and
+// G(i_k, c) + sum_{j<k} X_j(i_k) Y_j(c) gives Y_k into row(k) (j over the slots of
+// earlier sites).  Whole warps build the X rows, the next ones the Y columns.
+template <int NMAX, bool LEFT, bool PAIR>
 DEVI void block_vectors(const Ctx<NMAX>& x, const cplx* G, int n, int k0, int kb) {
-    constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD;
+    constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD, W = PAIR ? 2 : 1;
     const auto& s = x.s;
-    const cplx* xb = s.tau();
-    const cplx* yb = s.delta2();
-    for (int t = threadIdx.x; t < 2 * n; t += blockDim.x) {
-        const bool isx = t < n;
-        const int v = isx ? t : t - n;
+    const cplx *xb = s.xb(), *yb = s.yb();
+    const int ns = x.P().Ns;
+    const int n32 = (n + 31) & ~31;
+    kb = uni(kb);
+    for (int t = threadIdx.x; t < 2 * n32; t += blockDim.x) {
+        const bool isx = uni(t) < n32;
+        const int v = isx ? t : t - n32;
+        const int vc = min(v, n - 1);
+        const cplx* other = isx ? yb : xb;   // the other vector's values at the block's slots
         cplx acc[KB];
+        // the block's rows or columns of G first: their loads overlap
 #pragma unroll
         for (int k = 0; k < KB; ++k) {
-            if (k >= kb) break;
-            const int ik = LEFT ? n - 1 - (k0 + k) : k0 + k;
-            cplx a = isx ? G[v * LD + ik] : G[ik * LD + v];
+            const int ik = slot_index<LEFT, PAIR>(ns, k0, min(k, kb - 1));
+            acc[k] = G[isx ? vc * LD + ik : ik * LD + vc];
+        }
+        // a finished slot is added to all later ones at once (independent chains); slots from kb
+        // on take part with what the records hold and are stored as zeros
 #pragma unroll
-            for (int j = 0; j < k; ++j) a = isx ? cfma(acc[j], yb[j * KB + k], a) : cfma(xb[j * KB + k], acc[j], a);
-            if (isx) {
-                acc[k] = cmul(s.coef()[k], a);
-                s.col(k)[v] = acc[k];
+        for (int k = 0; k < KB; k += W) {
+            // X_k = coef g_k, or Y_k = e - g_k: one form for both, as a branch here would keep the
+            // loads of the later slots behind it
+            if constexpr (PAIR) {
+                const cplx* m = s.coef() + 2 * k;
+                const cplx ga = acc[k], gb = acc[k + 1];
+                const cplx xa = cfma(gb, m[2], cmul(ga, m[0])), xb_ = cfma(gb, m[3], cmul(ga, m[1]));
+                const double ea = v == slot_index<LEFT, PAIR>(ns, k0, k) ? 1.0 : 0.0;
+                const double eb = v == slot_index<LEFT, PAIR>(ns, k0, k + 1) ? 1.0 : 0.0;
+                acc[k] = cmk(isx ? xa.x : ea - ga.x, isx ? xa.y : -ga.y);
+                acc[k + 1] = cmk(isx ? xb_.x : eb - gb.x, isx ? xb_.y : -gb.y);
             } else {
-                acc[k] = cmk((v == ik ? 1.0 : 0.0) - a.x, -a.y);
-                s.row(k)[v] = acc[k];
+                const cplx c = s.coef()[k], xk = cmul(c, acc[k]);
+                const double e = v == slot_index<LEFT, PAIR>(ns, k0, k) ? 1.0 : 0.0;
+                acc[k] = cmk(isx ? xk.x : e - acc[k].x, isx ? xk.y : -acc[k].y);
             }
+#pragma unroll
+            for (int j = k; j < k + W; ++j)
+#pragma unroll
+                for (int l = k + W; l < KB; ++l) acc[l] = cfma(acc[j], other[j * KB + l], acc[l]);
+        }
+        cplx* dst = isx ? s.col(0) : s.row(0);
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+            const cplx w = cmk(k < kb ? acc[k].x : 0.0, k < kb ? acc[k].y : 0.0);
+            if (v < n) dst[k * Smem<NMAX>::VS + v] = w;
         }
     }
 }
 
-// Step 3 on one TR x TC tile at (r0, c0): G(r,c) += sum_m X_m(r) Y_m(c), then
-// (WRAP, the channel's last block) the deferred wrap.  Rejected slots have
-// X_m = 0 and add exact zeros; coef() is not read (the lead thread is already
-// writing the next block's coefficients).
-template <int NMAX, bool LEFT, bool WRAP>
-DEVI void rank_tile(const Ctx<NMAX>& x, cplx* G, int n, int kb, int r0, int c0) {
-    constexpr int TR = Cfg<NMAX>::TR, TC = Cfg<NMAX>::TC, KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD;
+// Step 3 on the FP64 tensor pipe, for the classes whose G is in shared memory: tiles of
+// 8 x 8 complex elements as in prod_mma, four mma per four slots, NB tiles of a warp in
+// flight; warp w of nw (the lead's scheduler excluded) takes contiguous tiles.  WRAP (the
+// channel's last block): the deferred wrap.  coef() is not read (the lead warp is already
+// writing the next block's).
+template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
+DEVI void rank_tiles(const Ctx<NMAX>& x, cplx* G, int n, int w, int nw, bool flip) {
+    constexpr int LD = Cfg<NMAX>::LD, KB = Cfg<NMAX>::KB, NB = 2;
     const auto& s = x.s;
-    cplx g[TR][TC];
+    n = uni(n);
+    w = uni(w);
+    const int lane = threadIdx.x & 31, l4 = lane & 3, l8 = lane >> 2;
+    const int n8 = (n + 7) >> 3, tiles = n8 * n8;
+    const int t1 = (w + 1) * tiles / nw;
+    int t0 = w * tiles / nw, rt = t0 / n8, ct = t0 - rt * n8;
+    for (; t0 < t1; t0 += NB) {
+        double re[NB][2], im[NB][2];
+        cplx a[NB][KB / 4], b[NB][KB / 4];
+        int r[NB], c[NB];
 #pragma unroll
-    for (int a = 0; a < TR; ++a)
+        for (int q = 0; q < NB; ++q) {
+            const int ra = min(tile_at(rt, l8), n - 1), cb = min(tile_at(ct, l8), n - 1);
+            r[q] = t0 + q < t1 ? tile_at(rt, l8) : n;
+            c[q] = 8 * ct + l4;
+            const cplx g0 = G[ra * LD + min(c[q], n - 1)], g1 = G[ra * LD + min(c[q] + 4, n - 1)];
+            re[q][0] = g0.x;
+            re[q][1] = g1.x;
+            im[q][0] = g0.y;
+            im[q][1] = g1.y;
 #pragma unroll
-        for (int b = 0; b < TC; ++b) g[a][b] = G[min(r0 + a, n - 1) * LD + min(c0 + b, n - 1)];
+            for (int k = 0; k < KB / 4; ++k) {
+                a[q][k] = s.col(4 * k + l4)[ra];   // slots from kb on hold zeros
+                b[q][k] = s.row(4 * k + l4)[cb];
+            }
+            const bool next = ++ct == n8;
+            ct = next ? 0 : ct;
+            rt = min(rt + (next ? 1 : 0), n8 - 1);
+        }
 #pragma unroll
-    for (int m = 0; m < KB; ++m) {
-        if (m >= kb) break;
-        cplx cr[TR], y[TC];
+        for (int k = 0; k < KB / 4; ++k) {
 #pragma unroll
-        for (int a = 0; a < TR; ++a) cr[a] = s.col(m)[min(r0 + a, n - 1)];
+            for (int q = 0; q < NB; ++q) {
+                mma_f64(re[q][0], re[q][1], a[q][k].x, b[q][k].x);
+                mma_f64(im[q][0], im[q][1], a[q][k].x, b[q][k].y);
+            }
 #pragma unroll
-        for (int b = 0; b < TC; ++b) y[b] = s.row(m)[min(c0 + b, n - 1)];
+            for (int q = 0; q < NB; ++q) {
+                mma_f64(re[q][0], re[q][1], -a[q][k].y, b[q][k].y);
+                mma_f64(im[q][0], im[q][1], a[q][k].y, b[q][k].x);
+            }
+        }
 #pragma unroll
-        for (int a = 0; a < TR; ++a)
-#pragma unroll
-            for (int b = 0; b < TC; ++b) g[a][b] = cfma(cr[a], y[b], g[a][b]);
-    }
-    if constexpr (WRAP) {
-        cplx fb[TC];
-#pragma unroll
-        for (int b = 0; b < TC; ++b) fb[b] = wrap_col<NMAX, LEFT>(s, min(c0 + b, n - 1));
-#pragma unroll
-        for (int a = 0; a < TR; ++a) {
-            const cplx fa = wrap_row<NMAX, LEFT>(s, min(r0 + a, n - 1));
-#pragma unroll
-            for (int b = 0; b < TC; ++b) g[a][b] = cmul(cmul(g[a][b], fa), fb[b]);
+        for (int q = 0; q < NB; ++q) {
+            cplx g0 = cmk(re[q][0], im[q][0]), g1 = cmk(re[q][1], im[q][1]);
+            if constexpr (WRAP) {
+                const cplx f = wrap_row<NMAX, LEFT, PAIR>(x, min(r[q], n - 1), flip);
+                g0 = cmul(cmul(g0, f), wrap_col<NMAX, LEFT, PAIR>(x, min(c[q], n - 1), flip));
+                g1 = cmul(cmul(g1, f), wrap_col<NMAX, LEFT, PAIR>(x, min(c[q] + 4, n - 1), flip));
+            }
+            if (r[q] < n && c[q] < n) G[r[q] * LD + c[q]] = g0;
+            if (r[q] < n && c[q] + 4 < n) G[r[q] * LD + c[q] + 4] = g1;
         }
     }
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-        for (int b = 0; b < TC; ++b)
-            if (r0 + a < n && c0 + b < n) G[(r0 + a) * LD + c0 + b] = g[a][b];
 }
 
 // Step 3 for the classes whose G lives in HBM/L2.  Items are (32-column chunk,
 // PR-row block): a warp's load or store of one row of an item is a coalesced
 // 512-byte segment.  Warp w (of nw, the lead's warp excluded) takes items
 // w, w + nw, ...
-template <int NMAX, bool LEFT, bool WRAP>
-DEVI void rank_rows(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw) {
+template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
+DEVI void rank_rows(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw, bool flip) {
     constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD, PR = 9;
     const auto& s = x.s;
     const int lane = threadIdx.x & 31;
@@ -686,9 +843,10 @@ DEVI void rank_rows(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw) {
             for (int a = 0; a < PR; ++a) g[a] = cfma(cr[min(rb + a, n - 1)], y, g[a]);
         }
         if constexpr (WRAP) {
-            const cplx fb = wrap_col<NMAX, LEFT>(s, c);
+            const cplx fb = wrap_col<NMAX, LEFT, PAIR>(x, c, flip);
 #pragma unroll
-            for (int a = 0; a < PR; ++a) g[a] = cmul(cmul(g[a], wrap_row<NMAX, LEFT>(s, min(rb + a, n - 1))), fb);
+            for (int a = 0; a < PR; ++a)
+                g[a] = cmul(cmul(g[a], wrap_row<NMAX, LEFT, PAIR>(x, min(rb + a, n - 1), flip)), fb);
         }
 #pragma unroll
         for (int a = 0; a < PR; ++a)
@@ -696,23 +854,47 @@ DEVI void rank_rows(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw) {
     }
 }
 
-template <int NMAX, bool LEFT>
+template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
+DEVI void rank_pass(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw, bool flip) {
+    if constexpr (Cfg<NMAX>::GG) rank_rows<NMAX, LEFT, PAIR, WRAP>(x, G, n, kb, w, nw, flip);
+    else rank_tiles<NMAX, LEFT, PAIR, WRAP>(x, G, n, w, nw, flip);
+}
+
+// Start the copy of a slice's fields (both channels) into shared memory: issued before the
+// products or the measurement that precede the slice's updates, which hide its latency.
+template <int NMAX>
+DEVI void stage_fields(const Ctx<NMAX>& x, int slice) {
+    const int ns = x.P().Ns;
+    const double* src = x.phi + (long)slice * ns * 2;
+    for (int i = threadIdx.x; i < ns; i += blockDim.x)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(x.s.fld() + 2 * i)),
+                     "l"(src + 2 * i)
+                     : "memory");
+}
+
+template <int NMAX, bool LEFT, bool PAIR>
 COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
-    constexpr int TR = Cfg<NMAX>::TR, TC = Cfg<NMAX>::TC, KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD;
+    constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD, W = PAIR ? 2 : 1, SB = KB / W;   // SB sites a block
     auto& s = x.s;
-    const int n = x.n, tid = threadIdx.x;
+    const int n = uni(x.n), ns = uni(x.P().Ns), tid = threadIdx.x;
+    x.sw0 = uni(x.sw0);
     const double ar = x.P().alpha_re[ch], ai = x.P().alpha_im[ch];
     const double shift = fabs(x.P().shiftLoc);
+    const bool flip = PAIR && x.P().flip[ch] != 0;
     const uint32_t s0 = *s.seed();
-    double* phis = x.phi + (long)slice * n * 2;
+    double* phis = x.phi + (long)slice * ns * 2;
     cplx* G = x.G();
 
-    // per-site proposals; draw order follows the visiting order of the sites
-    for (int i = tid; i < n; i += blockDim.x) {
-        const int m = LEFT ? (n - 1 - i) : i;
+    // the slice's fields were started on their way by stage_fields
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // per-site proposals (Nambu: opU_get_delta, src/pairing/src/operator_Hubbard.f90:100-137);
+    // draw order follows the visiting order of the sites
+    for (int i = tid; i < ns; i += blockDim.x) {
+        const int m = LEFT ? (ns - 1 - i) : i;
         const double xflip = lcg_u(lcg_mul(c_apow[2 * m + 1], s0));
         const double rnd = lcg_u(lcg_mul(c_apow[2 * m + 2], s0));
-        const double po = phis[i * 2 + ch];
+        const double po = s.fld()[i * 2 + ch];
         const double xdif = (xflip - 0.5) * shift;
         const double pn = po + xdif;
         const double go = exp(-0.5 * po * po), gn = exp(-0.5 * pn * pn);
@@ -723,252 +905,91 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
         s.ean()[i] = en;
         s.ebo()[i] = ebo;
         s.ebn()[i] = ebn;
-        s.delta()[i] = csub(ratio_unit(ar, ai, en, eo), cmk(1.0, 0.0));
-        s.rg()[i] = gn / go;
+        if constexpr (PAIR) {
+            cplx ep, em;
+            hs_factors(ar, ai, pn - po, ep, em);
+            const cplx dp = csub(ep, cmk(1.0, 0.0));
+            s.delta()[i] = dp;                                        // b_i: e^{+alpha dphi} - 1 in both channels
+            s.delta2()[i] = flip ? csub(em, cmk(1.0, 0.0)) : dp;      // c^dagger_i
+            // |ratio_gaussian * ratio_constant|; ratio_constant = e^{alpha(phi_old - phi_new)} for U2
+            const double rc = ch == 1 ? (ai == 0.0 ? fabs(eo.x / en.x) : cabsv(cdiv(eo, en))) : 1.0;
+            s.rg()[i] = (gn / go) * rc;
+        } else {
+            s.delta()[i] = csub(ratio_unit(ar, ai, en, eo), cmk(1.0, 0.0));
+            s.rg()[i] = gn / go;
+        }
         s.u2()[i] = rnd;
         s.phin()[i] = pn;
         s.accf()[i] = 0;
     }
     __syncthreads();
 
-    // Blocks of KB sites in visiting order.  The lead warp (warp sw0) decides
+    // Blocks of SB sites in visiting order.  The lead warp (warp sw0) decides
     // block b + 1 while the other warps run block b's rank pass: it
     // copies block b + 1's submatrix during block b's vector step (G is not
-    // written then) and adds block b's terms itself, exactly as the pass does.  The last block's pass applies the channel's deferred wrap.
+    // written then) and adds block b's terms itself.  The last block's pass applies
+    // the channel's deferred wrap.
     constexpr int NT = Cfg<NMAX>::THREADS;
     const bool lead = tid == 32 * x.sw0;
-    const int warp = tid >> 5;
+    const int warp = warp_index();
     const bool lwarp = warp == x.sw0;
-    const int rt = tid - (warp > x.sw0 ? 32 : 0);   // rank-pass thread index (lead warp excluded)
-    const int ncg = (n + TC - 1) / TC, ntiles = ncg * ((n + TR - 1) / TR);
+    // The lead's chain of dependent FP64 operations waits behind every mma (16 cycles) that
+    // another warp has on its scheduler (warp index modulo 4), so the pass leaves the
+    // schedulers of the leads alone: two of them with two CTAs on the SM, else one.
+    constexpr bool TWO = Cfg<NMAX>::LEADS == 2;
+    const int rel = (warp - x.sw0) & 3;
+    const int rw = TWO ? ((rel & 1) ? warp >> 1 : -1) : (rel ? (warp >> 2) * 3 + rel - 1 : -1);
+    constexpr int NRW = TWO ? NT / 64 : NT / 32 * 3 / 4;
     long long nacc = 0;   // accepted proposals, counted by the lead
     if (lwarp) {
-        block_snapshot<NMAX, LEFT>(s, G, n, 0, min(KB, n));
+        const int kb = W * min(SB, ns);
+        block_snapshot<NMAX, LEFT, PAIR>(x, G, 0, kb);
         __syncwarp();
-        const long long c = lead_block<NMAX, LEFT>(x, n, 0, min(KB, n), 0);
+        const long long c = lead_block<NMAX, LEFT, PAIR>(x, 0, kb, 0);
         if (lead) nacc += c;
     }
     __syncthreads();
-    for (int k0 = 0; k0 < n; k0 += KB) {
-        const int kb = min(KB, n - k0), k1 = k0 + KB, kb1 = min(KB, n - k1);
-        const bool more = k1 < n;
-        block_vectors<NMAX, LEFT>(x, G, n, k0, kb);
-        if (lwarp && more) block_snapshot<NMAX, LEFT>(s, G, n, k1, kb1);
+    for (int k0 = 0; k0 < ns; k0 += SB) {
+        const int kb = W * min(SB, ns - k0), k1 = k0 + SB, kb1 = W * min(SB, ns - k1);
+        const bool more = k1 < ns;
+        block_vectors<NMAX, LEFT, PAIR>(x, G, n, k0, kb);
+        if (lwarp && more) block_snapshot<NMAX, LEFT, PAIR>(x, G, k1, kb1);
         __syncthreads();
         if (lwarp) {
             if (more) {
-                const long long c = lead_block<NMAX, LEFT>(x, n, k1, kb1, kb);
+                const long long c = lead_block<NMAX, LEFT, PAIR>(x, k1, kb1, kb);
                 if (lead) nacc += c;
             }
-        } else if constexpr (Cfg<NMAX>::GG) {
-            const int w = warp - (warp > x.sw0 ? 1 : 0), nw = NT / 32 - 1;
-            if (more) rank_rows<NMAX, LEFT, false>(x, G, n, kb, w, nw);
-            else rank_rows<NMAX, LEFT, true>(x, G, n, kb, w, nw);
-        } else {
-            for (int tt = rt; tt < ntiles; tt += NT - 32) {
-                const int r0 = (tt / ncg) * TR, c0 = (tt % ncg) * TC;
-                if (more) rank_tile<NMAX, LEFT, false>(x, G, n, kb, r0, c0);
-                else rank_tile<NMAX, LEFT, true>(x, G, n, kb, r0, c0);
-            }
+        } else if (more) {
+            if (rw >= 0) rank_pass<NMAX, LEFT, PAIR, false>(x, G, n, kb, rw, NRW, flip);
+        } else if (rw >= 0) {
+            rank_pass<NMAX, LEFT, PAIR, true>(x, G, n, kb, rw, NRW, flip);
         }
         __syncthreads();
     }
     // accepted fields, counters, seed, and the U factor wrap with the final fields
-    for (int i = tid; i < n; i += blockDim.x)
-        if (s.accf()[i]) phis[i * 2 + ch] = s.phin()[i];
-    if (tid == 32 * x.sw0) {   // the lead thread: AccCounter%count, kept in shared memory
-        s.cnt()[ch] += nacc;
-        s.cnt()[2 + ch] += n;
-        *s.seed() = lcg_mul(c_apow[2 * n], s0);
-    }
-    {
-        constexpr int MAXE = Cfg<NMAX>::MAXE, T = Cfg<NMAX>::THREADS;
-        int r = tid / n, c = tid - (tid / n) * n;
-        const int dr = T / n, dc = T - (T / n) * n;
-#pragma unroll
-        for (int k = 0; k < MAXE; ++k) {
-            const int e = tid + k * T;
-            if (e < n * n) {
-                const int site = LEFT ? c : r;
-                const cplx f = s.accf()[site] ? s.ean()[site] : s.eao()[site];
-                x.U()[r * LD + c] = cmul(x.U()[r * LD + c], f);
-            }
-            c += dc;
-            r += dr;
-            if (c >= n) {
-                c -= n;
-                ++r;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// Nambu local update of one channel over all sites of one slice, fused with
-// the V-wrap of G (LocalU_prop_L / LocalU_prop_R and LocalU_metro,
-// src/pairing/src/localU.f90:33-149), on the {b, c^dagger} block.
-//
-// For site i the reference forms the 4x4 P = I + Delta (I - G[isec,isec]) over
-// the sectors b, c, b^dagger, c^dagger of the site, takes
-// ratio_det = det(P)^(-1/2), and on acceptance applies the rank-4 update
-// G -= G[:,isec] P^{-1} Delta (I[isec,:] - G[isec,:]).  With the block
-// structure P splits into the 2x2 block P1 on {b_i, c^dagger_i} and its
-// complex conjugate on {c_i, b^dagger_i}, so det(P) = |det P1|^2 (real and
-// positive: ratio_det = 1/|det P1|, and the ratio's phase that PhaseCounter
-// records is zero), and the update of the block is the rank-2 term
-// G1 -= G1[:,s] P1^{-1} D1 (I[s,:] - G1[s,:]), s = (i, Ns+i).
-//
-// Sites are sequential.  Every thread keeps the same MAXE elements of G in
-// registers for the whole slice; per site the owners of rows and columns i
-// and Ns+i stage them in shared memory (double-buffered by site parity), one
-// barrier, then every thread makes the same decision from the staged 2x2 and
-// updates its own elements.
-template <int NMAX, bool LEFT>
-COLD void prop_channel_pair(Ctx<NMAX> x, int ch, int slice) {
-    constexpr int MAXE = Cfg<NMAX>::MAXE, LD = Cfg<NMAX>::LD;
-    auto& s = x.s;
-    const int n = x.n, ns = x.P().Ns, tid = threadIdx.x;
-    const double ar = x.P().alpha_re[ch], ai = x.P().alpha_im[ch];
-    const double shift = fabs(x.P().shiftLoc);
-    const bool flip = x.P().flip[ch] != 0;
-    const bool total = (ch == 1);
-    const uint32_t s0 = *s.seed();
-    double* phis = x.phi + (long)slice * ns * 2;
-    cplx* G = x.G();
-
-    // per-site proposals (opU_get_delta, src/pairing/src/operator_Hubbard.f90:100-137)
-    for (int i = tid; i < ns; i += blockDim.x) {
-        const int m = LEFT ? (ns - 1 - i) : i;
-        const double xflip = lcg_u(lcg_mul(c_apow[2 * m + 1], s0));
-        const double rnd = lcg_u(lcg_mul(c_apow[2 * m + 2], s0));
-        const double po = phis[i * 2 + ch];
-        const double pn = po + (xflip - 0.5) * shift;
-        const double go = exp(-0.5 * po * po), gn = exp(-0.5 * pn * pn);
-        const cplx eo = cexpz(cmk(ar * po, ai * po)), en = cexpz(cmk(ar * pn, ai * pn));
-        const double dphi = pn - po;
-        const cplx dp = csub(cexpz(cmk(ar * dphi, ai * dphi)), cmk(1.0, 0.0));
-        const cplx dm = csub(cexpz(cmk(-(ar * dphi), -(ai * dphi))), cmk(1.0, 0.0));
-        s.eao()[i] = eo;
-        s.ean()[i] = en;
-        s.ebo()[i] = cexpz(cmk(-(ar * po), -(ai * po)));
-        s.ebn()[i] = cexpz(cmk(-(ar * pn), -(ai * pn)));
-        s.delta()[i] = dp;                  // b_i: e^{+alpha dphi} - 1 in both channels
-        s.delta2()[i] = flip ? dm : dp;     // c^dagger_i
-        // |ratio_gaussian * ratio_constant|; ratio_constant = e^{alpha(phi_old - phi_new)} for U2
-        const double rc = total ? cabsv(cdiv(eo, en)) : 1.0;
-        s.rg()[i] = (gn / go) * rc;
-        s.u2()[i] = rnd;
-        s.phin()[i] = pn;
-        s.accf()[i] = 0;
-    }
-    __syncthreads();
-
-    cplx g[MAXE];
-    int er[MAXE], ec[MAXE];
-    long long nacc = 0;   // accepted proposals, counted by thread 0
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = tid + k * blockDim.x;
-        er[k] = (e < n * n) ? e / n : -1;
-        ec[k] = (e < n * n) ? e - (e / n) * n : -1;
-        g[k] = (e < n * n) ? G[er[k] * LD + ec[k]] : cmk(0.0, 0.0);
-    }
-    for (int q = 0; q < ns; ++q) {
-        const int i = LEFT ? ns - 1 - q : q;
-        const int a = i, b = ns + i;
-        const int buf = (q & 1) * 2;
-        cplx* xa = s.col(buf);
-        cplx* xb = s.col(buf + 1);
-        cplx* ya = s.row(buf);
-        cplx* yb = s.row(buf + 1);
-        if (!LEFT) {   // opU_mmult_R(+1) then opU_mmult_L(-1) with the current field
-            const cplx ep = s.eao()[i], em = s.ebo()[i];
-#pragma unroll
-            for (int k = 0; k < MAXE; ++k) {
-                if (er[k] == a) g[k] = cmul(ep, g[k]);
-                else if (er[k] == b) g[k] = cmul(flip ? em : ep, g[k]);
-                if (ec[k] == a) g[k] = cmul(g[k], em);
-                else if (ec[k] == b) g[k] = cmul(g[k], flip ? ep : em);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < MAXE; ++k) {
-            if (ec[k] == a) xa[er[k]] = g[k];
-            if (ec[k] == b) xb[er[k]] = g[k];
-            if (er[k] == a) ya[ec[k]] = g[k];
-            if (er[k] == b) yb[ec[k]] = g[k];
-        }
-        __syncthreads();
-        // P1 = I + D1 (I - G1[s,s]);  accept if |rg rc| / |det P1| > u
-        const cplx d0 = s.delta()[i], d1 = s.delta2()[i];
-        const cplx gaa = ya[a], gab = ya[b], gba = yb[a], gbb = yb[b];
-        const cplx p00 = cadd(cmk(1.0, 0.0), cmul(d0, cmk(1.0 - gaa.x, -gaa.y)));
-        const cplx p01 = cmul(d0, cmk(-gab.x, -gab.y));
-        const cplx p10 = cmul(d1, cmk(-gba.x, -gba.y));
-        const cplx p11 = cadd(cmk(1.0, 0.0), cmul(d1, cmk(1.0 - gbb.x, -gbb.y)));
-        const cplx det = csub(cmul(p00, p11), cmul(p01, p10));
-        const double det2 = det.x * det.x + det.y * det.y;
-        const bool accept = s.rg()[i] / sqrt(det2) > s.u2()[i];
-        if (tid == 0) {
-            s.accf()[i] = accept ? 1 : 0;
-            nacc += accept ? 1 : 0;
-        }
-        if (accept) {
-            // M = P1^{-1} D1, P1^{-1} = adj(P1) conj(det) / |det|^2
-            const cplx id = cmk(det.x / det2, -det.y / det2);
-            const cplx m00 = cmul(cmul(p11, id), d0);
-            const cplx m01 = cmul(cmul(cmk(-p01.x, -p01.y), id), d1);
-            const cplx m10 = cmul(cmul(cmk(-p10.x, -p10.y), id), d0);
-            const cplx m11 = cmul(cmul(p00, id), d1);
-#pragma unroll
-            for (int k = 0; k < MAXE; ++k) {
-                if (er[k] < 0) continue;
-                const int r = er[k], c = ec[k];
-                const cplx ca = xa[r], cb = xb[r];
-                const cplx x0 = cadd(cmul(ca, m00), cmul(cb, m10));
-                const cplx x1 = cadd(cmul(ca, m01), cmul(cb, m11));
-                const cplx y0 = cmk(((c == a) ? 1.0 : 0.0) - ya[c].x, -ya[c].y);
-                const cplx y1 = cmk(((c == b) ? 1.0 : 0.0) - yb[c].x, -yb[c].y);
-                g[k] = csub(g[k], cadd(cmul(x0, y0), cmul(x1, y1)));
-            }
-        }
-        if (LEFT) {   // opU_mmult_L(+1) then opU_mmult_R(-1) with the final field
-            const cplx ep = accept ? s.ean()[i] : s.eao()[i];
-            const cplx em = accept ? s.ebn()[i] : s.ebo()[i];
-#pragma unroll
-            for (int k = 0; k < MAXE; ++k) {
-                if (ec[k] == a) g[k] = cmul(g[k], ep);
-                else if (ec[k] == b) g[k] = cmul(g[k], flip ? em : ep);
-                if (er[k] == a) g[k] = cmul(em, g[k]);
-                else if (er[k] == b) g[k] = cmul(flip ? ep : em, g[k]);
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k)
-        if (er[k] >= 0) G[er[k] * LD + ec[k]] = g[k];
-    __syncthreads();
     for (int i = tid; i < ns; i += blockDim.x)
-        if (s.accf()[i]) phis[i * 2 + ch] = s.phin()[i];
-    if (tid == 0) {
+        if (s.accf()[i]) phis[i * 2 + ch] = s.phin()[i];   // the other channel's staged values stay as they are
+    if (tid == 32 * x.sw0) {   // the lead thread: AccCounter%count, kept in shared memory
         s.cnt()[ch] += nacc;
         s.cnt()[2 + ch] += ns;
         *s.seed() = lcg_mul(c_apow[2 * ns], s0);
     }
-    // U_L columns (left) or U_R rows (right) of both indices of every site, final fields
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = tid + k * blockDim.x;
-        if (e < n * n) {
-            const int idx = LEFT ? ec[k] : er[k];
-            const int site = idx < ns ? idx : idx - ns;
+    {   // U_L columns (left) or U_R rows (right)
+        constexpr int MAXE = Cfg<NMAX>::MAXE, T = Cfg<NMAX>::THREADS;
+        const uint32_t dm = div_magic(n);
+        cplx* U = x.U();
+#pragma unroll 3
+        for (int k = 0; k < MAXE; ++k) {
+            const int e = min(tid + k * T, n * n - 1);   // the last threads repeat the last element without storing it
+            const int r = div_by(e, dm), c = e - r * n;
+            const int idx = LEFT ? c : r;
+            const bool cd = PAIR && idx >= ns;
+            const int site = cd ? idx - ns : idx;
             const bool acc = s.accf()[site] != 0;
-            const cplx ep = acc ? s.ean()[site] : s.eao()[site];
-            const cplx em = acc ? s.ebn()[site] : s.ebo()[site];
-            const cplx f = (idx >= ns && flip) ? em : ep;
-            cplx* u = x.U() + er[k] * LD + ec[k];
-            *u = LEFT ? cmul(*u, f) : cmul(f, *u);
+            const cplx* f = cd && flip ? (acc ? s.ebn() : s.ebo()) : (acc ? s.ean() : s.eao());
+            const cplx v = cmul(U[r * LD + c], f[site]);
+            if (tid + k * T < n * n) U[r * LD + c] = v;
         }
     }
     __syncthreads();
@@ -984,14 +1005,14 @@ COLD void slice_products(Ctx<NMAX> x) {
     const int n = x.n;
     const double* P = reinterpret_cast<const double*>(x.W1());   // e^{-dtau K}, real
     const double* M = reinterpret_cast<const double*>(x.W2());   // e^{+dtau K}, real
-    if (LEFT) {
-        slice_mult<NMAX, true>(x, x.G(), P);
-        slice_mult<NMAX, false>(x, x.G(), M);
-        slice_mult<NMAX, true>(x, x.U(), P);
+    // G and U take the same first factor: one call for both where the products run in place
+    if constexpr (Cfg<NMAX>::GG) {
+        slice_mult<NMAX, LEFT>(x, x.G(), P);
+        slice_mult<NMAX, !LEFT>(x, x.G(), M);
+        slice_mult<NMAX, LEFT>(x, x.U(), P);
     } else {
-        slice_mult<NMAX, false>(x, x.G(), P);
-        slice_mult<NMAX, true>(x, x.G(), M);
-        slice_mult<NMAX, false>(x, x.U(), P);
+        gemm_real_any<NMAX, LEFT>(x, x.G(), P, x.U());
+        gemm_real_any<NMAX, !LEFT>(x, x.G(), M);
     }
 }
 
@@ -1017,9 +1038,10 @@ COLD void measure(Ctx<NMAX> x) {
 #pragma unroll
     for (int k = 0; k < 14; ++k) v[k] = 0.0;
     const int* sxy = s.sxy();
-    const int T = blockDim.x, di = T / n, dj = T - (T / n) * n;
-    int i = tid / n, j = tid - (tid / n) * n;
+    const int T = blockDim.x;
+    const uint32_t dm = div_magic(n);
     for (int e = tid; e < n * n; e += T) {
+        const int i = div_by(e, dm), j = e - i * n;
         const cplx a = G[i * LD + j];                 // Grup(i,j)
         cplx gc = G[j * LD + i];                      // Grupc(i,j) = G(j,i) - delta_ij
         if (i == j) gc.x -= 1.0;
@@ -1045,12 +1067,6 @@ COLD void measure(Ctx<NMAX> x) {
             v[3] += p.y * sfr;
             v[4] += p.x * dwr;
             v[5] += p.y * dwr;
-        }
-        j += dj;
-        i += di;
-        if (j >= n) {
-            j -= n;
-            ++i;
         }
     }
     for (int e = tid; e < 3 * n; e += blockDim.x) {   // bonds (x+1,y), (x,y+1), (x-1,y+1) (lattice.f90:98-111)
@@ -1133,9 +1149,10 @@ COLD void measure_pair(Ctx<NMAX> x) {
 #pragma unroll
     for (int k = 0; k < 19; ++k) v[k] = 0.0;
     const int* sxy = s.sxy();
-    const int T = blockDim.x, stepi = T / ns, stepj = T - (T / ns) * ns;
-    int i = tid / ns, j = tid - (tid / ns) * ns;
+    const int T = blockDim.x;
+    const uint32_t dm = div_magic(ns);
     for (int e = tid; e < ns * ns; e += T) {
+        const int i = div_by(e, dm), j = e - i * ns;
         const cplx A = G[i * LD + j], B = G[i * LD + ns + j], C = G[(ns + i) * LD + j], D = G[(ns + i) * LD + ns + j];
         const cplx di = G[(ns + i) * LD + ns + i], dj = G[(ns + j) * LD + ns + j];
         const cplx nbi = cmk(-di.x, di.y), nbj = cmk(-dj.x, dj.y), ncj = cmk(-dj.x, -dj.y);
@@ -1158,12 +1175,6 @@ COLD void measure_pair(Ctx<NMAX> x) {
             v[6] += p.y * sfr;
             v[7] += p.x * dwr;
             v[8] += p.y * dwr;
-        }
-        j += stepj;
-        i += stepi;
-        if (j >= ns) {
-            j -= ns;
-            ++i;
         }
     }
     for (int e = tid; e < 3 * ns; e += blockDim.x) {   // bonds (x+1,y), (x,y+1), (x-1,y+1)
@@ -1251,15 +1262,16 @@ COLD void stab_UR(Ctx<NMAX> x) {
     constexpr int LD = Cfg<NMAX>::LD;
     auto& s = x.s;
     const int n = x.n;
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         x.W1()[r * LD + c] = cmul(x.U()[r * LD + c], x.A().DRc[c]);
     }
     __syncthreads();
     qrp_any(x, x.W1());
     for (int i = threadIdx.x; i < n; i += blockDim.x) x.A().DRc[i] = cmk(s.d()[i], 0.0);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         x.W2()[r * LD + c] = x.A().VRc[s.piv()[r] * n + c];
     }
     __syncthreads();
@@ -1275,15 +1287,16 @@ COLD void stab_UL(Ctx<NMAX> x) {
     constexpr int LD = Cfg<NMAX>::LD;
     auto& s = x.s;
     const int n = x.n;
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         x.W1()[r * LD + c] = cmul(cconj(x.U()[c * LD + r]), x.A().DLc[c]);
     }
     __syncthreads();
     qrp_any(x, x.W1());
     for (int i = threadIdx.x; i < n; i += blockDim.x) x.A().DLc[i] = cmk(s.d()[i], 0.0);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         x.W2()[r * LD + c] = x.A().VLc[r * n + s.piv()[c]];
     }
     __syncthreads();
@@ -1356,8 +1369,9 @@ DEVI void form_M(Ctx<NMAX>& x) {
     constexpr int LD = Cfg<NMAX>::LD;
     auto& s = x.s;
     const int n = x.n;
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         const cplx t = cmul(x.A().DLc[c], x.W1()[r * LD + c]);
         x.W2()[r * LD + c] = csub(x.W2()[r * LD + c], cmul(x.A().DRc[r], t));
     }
@@ -1369,10 +1383,11 @@ template <int NMAX>
 DEVI void drift_and_replace(Ctx<NMAX>& x) {
     auto& s = x.s;
     const int n = x.n;
+    const uint32_t dm = div_magic(n);
     double v[1] = {0.0};
     constexpr int LD = Cfg<NMAX>::LD;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - (e / n) * n;
+        const int r = div_by(e, dm), c = e - r * n;
         v[0] += cabsv(csub(x.W2()[r * LD + c], x.G()[r * LD + c]));
     }
     block_sum<1>(v, s.red());
@@ -1473,11 +1488,12 @@ DEVI bool setup_ctx(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
         *x.s.P() = ka.pts[cd.point];
         // The SM's schedulers take warps by slot modulo 4, so the deciding warps
         // of two CTAs on one SM would share a scheduler if both used warp 0.  A
-        // CTA whose warp slots start at an odd multiple of 8 decides on warp 2.
+        // CTA whose warp slots start at an odd multiple of 8 decides on warp 2; the
+        // four-warp CTAs, several to an SM, take the warp of their place among four.
         // Thread 0 decides for the whole CTA.
         unsigned slot;
         asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
-        *x.s.strip_warp() = (Cfg<NMAX>::THREADS >= 192 && ((slot >> 3) & 1)) ? 2 : 0;
+        *x.s.strip_warp() = Cfg<NMAX>::THREADS >= 192 ? (((slot >> 3) & 1) ? 2 : 0) : (slot >> 2) & 3;
     }
     __syncthreads();
     x.n = x.P().N;
@@ -1506,8 +1522,7 @@ DEVI void flush_obs(Ctx<NMAX>& x, double* gobs) {
 
 template <int NMAX, bool PAIR, bool LEFT>
 DEVI void prop_any(Ctx<NMAX>& x, int ch, int slice) {
-    if constexpr (PAIR) prop_channel_pair<NMAX, LEFT>(x, ch, slice);
-    else prop_channel<NMAX, LEFT>(x, ch, slice);
+    prop_channel<NMAX, LEFT, PAIR>(x, ch, slice);
 }
 template <int NMAX, bool PAIR>
 DEVI void measure_any(Ctx<NMAX>& x) {
@@ -1554,6 +1569,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) sweep_ker
                 wrap_L(x, nt);
                 lap(3);
             }
+            stage_fields(x, nt - 1);
             measure_any<NMAX, PAIR>(x);
             lap(2);
             slice_products<NMAX, true>(x);
@@ -1572,10 +1588,12 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) sweep_ker
     __syncthreads();
     wrap_R(x, 0);
     lap(3);
+    stage_fields(x, 0);
     for (int nt = 1; nt <= L; ++nt) {
         if (x.P().active[0]) prop_any<NMAX, PAIR, false>(x, 0, nt - 1);
         if (x.P().active[1]) prop_any<NMAX, PAIR, false>(x, 1, nt - 1);
         lap(0);
+        if (nt < L) stage_fields(x, nt);
         slice_products<NMAX, false>(x);
         lap(1);
         if (nt % x.P().Nwrap == 0) {
@@ -1616,6 +1634,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
     tc_begin(x, ka);
     auto& s = x.s;
     const int n = x.n, L = x.P().L;
+    const uint32_t dm = div_magic(n);
     set_identity(n, LD, x.U());
     set_identity(n, LD, x.G());
     set_identity(n, n, x.A().VRc);
@@ -1629,7 +1648,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
     sstore(n, LD, x.A().URs(0), x.U());
     gcopy(x.A().VRs(0), x.A().VRc, n * n);
     gcopy(x.A().DRs(0), x.A().DRc, n);
-    sload_real(n, LD, reinterpret_cast<double*>(x.W1()), x.P().expP);
+    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
     __syncthreads();
     const int ns = x.P().Ns;
     for (int nt = 1; nt <= L; ++nt) {
@@ -1639,7 +1658,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
             const double ar = x.P().alpha_re[ch], ai = x.P().alpha_im[ch];
             const bool flip = x.P().flip[ch] != 0;
             for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-                const int r = e / n, c = e - (e / n) * n;
+                const int r = div_by(e, dm), c = e - r * n;
                 const int site = (PAIR && r >= ns) ? r - ns : r;
                 const double p = ph[site * 2 + ch];
                 const bool neg = PAIR && r >= ns && flip;
@@ -1661,7 +1680,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
                 scopy(n, LD, x.G(), x.W2());
                 __syncthreads();
             }
-            sload_real(n, LD, reinterpret_cast<double*>(x.W1()), x.P().expP);
+            sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
             __syncthreads();
         }
     }
@@ -1972,8 +1991,9 @@ COLD void tau_solve(Ctx<NMAX>& x, cplx* A, cplx* C) {
 
 template <int NMAX>
 DEVI void tau_copy(int n, cplx* dst, const cplx* src) {   // both with the class's leading dimension
+    const uint32_t dm = div_magic(n);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - r * n;
+        const int r = div_by(e, dm), c = e - r * n;
         dst[r * taud::LD<NMAX> + c] = src[r * taud::LD<NMAX> + c];
     }
     __syncthreads();
@@ -1983,9 +2003,10 @@ DEVI void tau_copy(int n, cplx* dst, const cplx* src) {   // both with the class
 // valid in thread 0
 template <int NMAX>
 DEVI double tau_l1(Ctx<NMAX>& x, int n, const cplx* a, const cplx* b) {
+    const uint32_t dm = div_magic(n);
     double v[1] = {0.0};
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - r * n;
+        const int r = div_by(e, dm), c = e - r * n;
         const cplx d = csub(a[r * taud::LD<NMAX> + c], b[r * taud::LD<NMAX> + c]);
         v[0] += sqrt(d.x * d.x + d.y * d.y);
     }
@@ -2000,6 +2021,7 @@ template <int NMAX>
 COLD void tau_slice(Ctx<NMAX>& x, int nt) {
     constexpr int LD = taud::LD<NMAX>;
     const int n = x.n;
+    const uint32_t dm = div_magic(n);
     const PointDev& P = x.P();
     cplx *T0 = taud::slot(x, taud::GT0), *T1 = taud::slot(x, taud::G0T), *T2 = taud::slot(x, taud::GTT);
     cplx* U = x.U();
@@ -2020,7 +2042,7 @@ COLD void tau_slice(Ctx<NMAX>& x, int nt) {
         }
         __syncthreads();
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-            const int r = e / n, c = e - r * n;
+            const int r = div_by(e, dm), c = e - r * n;
             T0[r * LD + c] = cmul(ep[r], T0[r * LD + c]);
             T1[r * LD + c] = cmul(T1[r * LD + c], em[c]);
             T2[r * LD + c] = cmul(cmul(ep[r], T2[r * LD + c]), em[c]);
@@ -2030,11 +2052,9 @@ COLD void tau_slice(Ctx<NMAX>& x, int nt) {
     }
     const double *kp = reinterpret_cast<const double*>(taud::slot(x, taud::EP)),
                  *km = reinterpret_cast<const double*>(taud::slot(x, taud::EM));
-    gemm_real_any<NMAX, false>(x, T0, kp, T0);
-    gemm_real_any<NMAX, true>(x, T1, T1, km);
-    gemm_real_any<NMAX, false>(x, T2, kp, T2);
-    gemm_real_any<NMAX, true>(x, T2, T2, km);
-    gemm_real_any<NMAX, false>(x, U, kp, U);
+    gemm_real_any<NMAX, false>(x, T0, kp, T2);
+    gemm_real_any<NMAX, true>(x, T1, km, T2);
+    gemm_real_any<NMAX, false>(x, U, kp);
 }
 
 // Wrap_tau at slice nt (stabilization.f90:368-404): stab_UR of the propagated
@@ -2107,18 +2127,19 @@ COLD void tau_pass(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
     using namespace taud;
     constexpr int LD = taud::LD<NMAX>;
     const int n = x.n, L = x.P().L;
+    const uint32_t dm = div_magic(n);
     const Arena A = x.A();
     cplx *G = x.G(), *T0 = slot(x, GT0), *T1 = slot(x, G0T), *T2 = slot(x, GTT);
     cplx *sv = slot(x, VEC), *svr = slot(x, VR);
     gcopy(sv, A.DRc, n);
     gcopy(svr, A.VRc, n * n);
-    sload_real(n, LD, reinterpret_cast<double*>(slot(x, EP)), x.P().expP);
-    sload_real(n, LD, reinterpret_cast<double*>(slot(x, EM)), x.P().expM);
+    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(slot(x, EP)), x.P().expP);
+    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(slot(x, EM)), x.P().expM);
     sload(n, LD, G, A.G);
     sload(n, LD, x.U(), A.URc);
     __syncthreads();
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = e / n, c = e - r * n;
+        const int r = div_by(e, dm), c = e - r * n;
         const cplx g = G[r * LD + c];
         T0[r * LD + c] = g;
         T2[r * LD + c] = g;
