@@ -23,7 +23,7 @@ LIB = PKG / "libbafqmc_b200.so"
 STAMP = PKG / "libbafqmc_b200.so.sha256"
 OBJDIR = PKG.parent / "_build"
 SOURCES = ["sweep_kernels.cu", "pole_kernels.cu", "proposer.cu", "capi.cu"]
-HEADERS = ["cplx.cuh", "mma64.cuh", "linalg.cuh", "linalg_big.cuh", "tc.cuh", "sweep.cuh", "kernels.h", "net.h", "conv_tc.cuh"]
+HEADERS = ["cplx.cuh", "mma64.cuh", "linalg.cuh", "linalg_big.cuh", "tc.cuh", "sweep.cuh", "kernels.h", "net.h", "conv_tc.cuh", "wgrad_mma.cuh"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",

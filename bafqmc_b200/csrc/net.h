@@ -83,6 +83,7 @@ struct bafqmc_net {
     int* d_pairs = nullptr;      // [2 * cap] (input, target) configuration indices of a training batch
     uint64_t train_counter = 0;
     int use_tc = 1;              // convolutions on the tensor cores (where conv_tc_applies)
+    int wgrad_tc = 1;            // weight gradients on the tensor cores (where wgrad_mma_applies)
     int* d_err = nullptr;        // status of the tensor-core kernels (bounded waits that expired)
     int wait_test = 0;           // bafqmc_net_set_wait_test: MMAs skipped, short wait bound
     // proposal bookkeeping of the move: log q(phi'|phi) and the Hastings term per chain

@@ -14,7 +14,8 @@
 //
 // Kernels here run on the CUDA cores and serve every layer shape; every layer
 // of the forward pass and of the input-gradient pass also has a tensor-core
-// path (conv_tc.cuh) for width 64, sites a multiple of 4 and L a multiple of 32.
+// path (conv_tc.cuh) for width 64, sites a multiple of 4 and L a multiple of 32, and
+// the weight gradients of a width-64 network one for every lattice (wgrad_mma.cuh).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -24,6 +25,7 @@
 #include "conv_tc.cuh"
 #include "net.h"
 #include "sweep.cuh"
+#include "wgrad_mma.cuh"
 
 namespace bq {
 
@@ -536,23 +538,28 @@ cudaError_t net_backward(bafqmc_net* n, int chains) {
     const int nchunk = (int)std::min<long long>(256, (npts + 2047) / 2048);
     const long long per = ((npts + nchunk - 1) / nchunk + 31) / 32 * 32;
     for (int l = kNetLayers - 1; l >= 0 && e == cudaSuccess; --l) {
-        WgradArgs w{};
-        w.s = s;
-        w.x = n->d_act[l];
-        w.pin = s.pin[l];
-        w.cin = s.cin[l];
-        w.g = n->d_gact[l];
-        w.pout = s.pout[l];
-        w.cout = s.cout[l];
-        w.dw = n->d_grad + s.woff[l];
-        w.npts = npts;
-        w.per = per;
-        wgrad_ref_kernel<<<dim3(kNetTaps, nchunk), 256, 0, n->stream>>>(w);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) break;
-        bgrad_kernel<<<nchunk, 256, 0, n->stream>>>(s, n->d_gact[l], s.pout[l], s.cout[l], n->d_grad + s.boff[l], npts,
-                                                    per);
-        e = cudaGetLastError();
+        if (n->wgrad_tc && wgrad_mma_applies(s, l)) {
+            e = launch_wgrad_mma(s, l, chains, n->d_act[l], n->d_gact[l], n->d_grad + s.woff[l], n->d_grad + s.boff[l],
+                                 n->stream);
+        } else {
+            WgradArgs w{};
+            w.s = s;
+            w.x = n->d_act[l];
+            w.pin = s.pin[l];
+            w.cin = s.cin[l];
+            w.g = n->d_gact[l];
+            w.pout = s.pout[l];
+            w.cout = s.cout[l];
+            w.dw = n->d_grad + s.woff[l];
+            w.npts = npts;
+            w.per = per;
+            wgrad_ref_kernel<<<dim3(kNetTaps, nchunk), 256, 0, n->stream>>>(w);
+            e = cudaGetLastError();
+            if (e != cudaSuccess) break;
+            bgrad_kernel<<<nchunk, 256, 0, n->stream>>>(s, n->d_gact[l], s.pout[l], s.cout[l], n->d_grad + s.boff[l],
+                                                        npts, per);
+            e = cudaGetLastError();
+        }
         if (e != cudaSuccess || l == 0) break;
         if (n->use_tc && conv_tc_applies(s, l, true))
             e = launch_conv_tc(n, l, true, chains);
@@ -861,7 +868,7 @@ int bafqmc_net_set_tensor_cores(bafqmc_net* n, int enable) {
     if (enable && !bq::conv_tc_applies(n->shape, 1, false))
         return bq::net_fail(BAFQMC_EUNSUPPORTED,
                             "the tensor-core convolution needs width 64, sites a multiple of 4 and Ltrot a multiple of 32");
-    n->use_tc = enable ? 1 : 0;
+    n->use_tc = n->wgrad_tc = enable ? 1 : 0;
     return BAFQMC_OK;
 }
 
