@@ -76,6 +76,7 @@ struct bafqmc_net {
     double* d_losses = nullptr;  // per training step
     int losses_cap = 0;
     float* d_tin = nullptr;      // host-supplied configurations (float32) of the test entry points
+    float* h_tin = nullptr;      // pinned host side of it
     long long tin_cap = 0;
     // training set: configurations of the plain sampler, float32 [slot][chain][L][Ns][2]
     float* d_data = nullptr;
