@@ -54,6 +54,14 @@ DEVI double rcp_fast(double x) {
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
+// 1 / sqrt(x) likewise: the approximation and the third-order step
+// y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2, for normal x > 0.
+DEVI double rsqrt_fast(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y, e * fma(0.375, e, 0.5), y);
+}
 // exp(z) for complex z
 DEVI cplx cexpz(cplx z) {
     double s, c;

@@ -135,190 +135,254 @@ struct QRScratch {
     double* d;      // n   |R_ii|
     cplx* bcast;    // 4   broadcast slots
     int* ibcast;    // 4
+    // qr_columns only, in buffers of the local update
+    cplx* vb;         // n   the pivot column
+    cplx* scl;        // n   1 / d of the reflectors
+    long long* keys;  // n   remaining norms of the columns as ordered integers
+    double* bet;      // n   signed diagonal of R
+    int* ex;          // n   scale exponents of the columns
 };
 
-// ZGEQP3 (unblocked ZLAQP2 recurrence) on A (n x n) followed by the reference's
-// QDRP_decompose post-step (stabilization.f90:41-67): d[i] = |R_ii| and row i of
-// the upper triangle divided by d[i].  On exit A holds the scaled R in its upper
-// triangle and the Householder vectors (unit leading entry implicit) below it.
+// Scale 2^e of a column by its largest entry, as an exponent: 0 for a zero or non-finite column.
+DEVI int scale_exponent(double m) {
+    const int e = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
+    return (e == 0 || e == 0x7ff) ? 0 : e - 1022;
+}
+
+// Pivoted QR of A (n x n): (A P) = Q R with ZGEQP3's pivot rule (the column of largest
+// remaining norm), then the reference's QDRP_decompose post-step (stabilization.f90:41-67):
+// d[i] = |R_ii| and row i of the upper triangle divided by d[i], piv and ipiv.
+// AUG: also out <- Q^H in for the n x n view `in` (the identity if in.p is null), carried
+// along with the columns of A, so that no pass over the reflectors follows; A's strict
+// lower triangle is then not written.  Otherwise A holds the Householder vectors (unit
+// leading entry implicit) below R, and s.tau their factors, for form_q and apply_*.
 //
-// Two barriers per column.  Every warp finds the pivot (IDAMAX of the partial
-// norms) and every 8-lane segment forms the reflector (ZLARFG) itself from the
-// pivot column, so neither needs a barrier of its own; each segment keeps its
-// target columns in registers from the read phase to the write phase.  The
-// norm downdate is ZLAQP2's, with its quotients multiplied out (no division).
-// R8 >= ceil(n/8) rows per lane, CPS >= ceil(n/segments) columns per segment.
-template <int R8, int CPS>
-COLD void qrp_inplace(int n, int ld, cplx* A, QRScratch s) {
-    const uint32_t dm = div_magic(n);
-    const int tid = threadIdx.x, lane = tid & 31, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    const double tol3z = 1.0536712127723509e-08;   // sqrt(2^-53), LAPACK's sqrt(dlamch('E'))
-    for (int j = seg; j < n; j += nseg) {
-        const double v = seg8_norm(n, ld, A, j, 0, lane8);
-        if (lane8 == 0) { s.vn1[j] = v; s.vn2[j] = v; s.piv[j] = j; }
-    }
-    __syncthreads();
-    for (int i = 0; i < n; ++i) {
-        // pivot: first index of max vn1[i..n) (IDAMAX), every warp
-        double best = -1.0;
-        int bi = n;
-        for (int j = i + lane; j < n; j += 32) {
-            const double v = s.vn1[j];
-            if (v > best) { best = v; bi = j; }
-        }
+// LPC lanes own a column for the whole factorisation, RPL of its rows each in registers
+// (RPL * LPC >= n), with the same lanes for a column of `in`; pivoting is by bookkeeping,
+// no column moves, and a column is written once, at its place.  Per step the warps that
+// own columns (a named barrier, the others wait at the end) choose the pivot from the
+// keys in shared memory (redux on their bits), its owner copies it to shared memory, and
+// every group forms the reflector for itself: its norm is the sum of squares of the
+// column that the previous step's update left (every step computes the remaining norms
+// exactly, so ZLAQP2's downdating and its recomputation test are not needed), and the
+// product of the unscaled reflector with a column is under way while sqrt and 1/x are.
+// Columns are scaled by powers of two on entry (exact, and reflectors act on rows), so
+// that no sum of squares over- or underflows whatever D has grown to.
+// Rows leave the registers from the top, a block of LPC at a time, so that no step masks
+// them; a branch or a select per row cost more than the arithmetic (3500 cycles a step).
+// Bound: the chain and the issue of a step on the warps that own columns, 1860 cycles at
+// n = 36 with the second matrix (1460 without, 1075 at n = 16); 139 K -> 67 K cycles for the
+// factorisation.  The version before kept the matrix in shared memory, reduced over eight
+// lanes, downdated the norms and applied the reflectors in a pass of its own: a wrap of a
+// 36-site chain took 560 K cycles with that one and takes 270 K.
+// The per-thread state of the factorisation: its rows of the column of A and of `in`.
+template <int RPL, bool AUG>
+struct QrCol {
+    cplx a[RPL], c[AUG ? RPL : 1];
+    double n2;
+    int ex;
+    bool live;
+};
+
+// The LPC steps of row block kb, with K register rows left (those past n hold zeros).
+template <int LPC, int RPL, int K, bool AUG>
+DEVI void qr_block(int n, int ld, int kb, int nthr, cplx* A, const QRScratch& s, QrCol<RPL, AUG>& q, cplx* o, int osr,
+                   int ocj) {
+    constexpr long long kOff = (long long)0x8000000000000000ull;
+    const int tid = threadIdx.x, lane = tid & 31, lc = tid % LPC, j = tid / LPC, lj = min(lane, n - 1);
+    const bool first = lc == 0 && j < n;
+    const auto group_sum = [&](double v) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        const int pvt = (bi < n) ? bi : i;   // all-NaN norms: keep column i
-        // reflector of the pivot column (ZLARFG), every segment
-        cplx v[R8];
-        double ss = 0.0;
+        for (int d = LPC / 2; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        return v;
+    };
+#pragma unroll 1
+    for (int li = 0; li < LPC; ++li) {
+        const int i = kb * LPC + li, src = (lane & ~(LPC - 1)) + li;
+        if (i >= n) break;
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        // pivot: the largest key, the lowest column of equal ones (every warp for itself)
+        long long key = s.keys[lj];
+        int bj = lj;
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = lane8 + 8 * k;
-            v[k] = (r < n && r > i) ? A[r * ld + pvt] : cmk(0.0, 0.0);
-            ss = fma(v[k].x, v[k].x, fma(v[k].y, v[k].y, ss));
+        for (int w = 32; w < LPC * RPL; w += 32) {
+            const int jq = min(lane + w, n - 1);
+            const long long k2 = s.keys[jq];
+            bj = k2 > key ? jq : bj;
+            key = k2 > key ? k2 : key;
         }
-        ss = seg8_sum(ss);
-        const cplx alpha = A[i * ld + pvt];
-        double xn = sqrt(ss);
-        if (sumsq_unsafe(ss)) xn = seg8_colnorm(n, ld, A, pvt, i + 1, lane8);
-        cplx tau = cmk(0.0, 0.0), beta = alpha, scl = cmk(0.0, 0.0);
-        if (!(xn == 0.0 && alpha.y == 0.0)) {
-            const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn * xn);
-            const double b = (alpha.x >= 0.0) ? -nrm : nrm;
-            const double ib = 1.0 / b;
-            tau = cmk((b - alpha.x) * ib, -alpha.y * ib);
-            const cplx d = cmk(alpha.x - b, alpha.y);           // scl = 1 / d
-            const double id2 = 1.0 / (d.x * d.x + d.y * d.y);
-            scl = cmk(d.x * id2, -d.y * id2);
-            beta = cmk(b, 0.0);
+        const int hi = (int)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+        const int p = (int)__reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)bj : 0x7fffffffu);
+        const bool own = q.live && j == p;
+        q.live = q.live && !own;
+        const double pn = s.vn1[p];
+        if (own) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) s.vb[lc + LPC * k] = q.a[k];
         }
+        // row i leaves the registers
+        const cplx ai = cmk(__shfl_sync(0xffffffffu, q.a[0].x, src), __shfl_sync(0xffffffffu, q.a[0].y, src));
+        cplx ci = cmk(0.0, 0.0);
+        if constexpr (AUG) ci = cmk(__shfl_sync(0xffffffffu, q.c[0].x, src), __shfl_sync(0xffffffffu, q.c[0].y, src));
+        const bool at = lc == li;
+        q.a[0] = cmk(at ? 0.0 : q.a[0].x, at ? 0.0 : q.a[0].y);
+        if constexpr (AUG) q.c[0] = cmk(at ? 0.0 : q.c[0].x, at ? 0.0 : q.c[0].y);
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        const cplx alpha = s.vb[li];
+        // S = sum over rows below i of conj(x) a, in two chains each
+        constexpr bool KEEP = K * (AUG ? 3 : 2) <= 20;   // else read again below: the registers are full
+        cplx x[KEEP ? K : 1], sa[2], sc[2];
+        sa[0] = sa[1] = sc[0] = sc[1] = cmk(0.0, 0.0);
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = lane8 + 8 * k;
-            v[k] = (r == i) ? cmk(1.0, 0.0) : cmul(scl, v[k]);
+        for (int k = 0; k < K; ++k) {
+            const cplx xk = s.vb[lc + LPC * k];
+            if constexpr (KEEP) x[k] = xk;
+            sa[k & 1] = cfmacj(xk, q.a[k], sa[k & 1]);
+            if constexpr (AUG) sc[k & 1] = cfmacj(xk, q.c[k], sc[k & 1]);
         }
-        // target columns j = i+1+seg+q*nseg; logical column pvt holds the old column i
-        cplx a[CPS][R8];
-        double t1[CPS], t2[CPS];
+        // beta = b = -sign(Re alpha) |column|, d = alpha - b, tau = (b - alpha) / b = -d / b (ZLARFG);
+        // the unscaled reflector (d, x) takes conj(tau) / |d|^2 = -conj(d) / (b |d|^2)
+        const bool zero = !(pn > 1.0e-300);
+        const double y = rsqrt_fast(zero ? 1.0 : pn), nrm = pn * y;
+        const double b = alpha.x >= 0.0 ? -nrm : nrm;
+        const cplx d = cmk(alpha.x - b, alpha.y);
+        const double d2 = fma(d.x, d.x, d.y * d.y);
+        const double t0 = rcp_fast(b * d2), t = zero ? 0.0 : t0;
+        const cplx tq = cmk(d.x * t, -d.y * t);   // minus the factor
+        const cplx wa = cfmacj(d, ai, cmk(group_sum(sa[0].x + sa[1].x), group_sum(sa[0].y + sa[1].y)));
+        const cplx f = cmul(tq, wa);
+        const cplx fa = cmk(q.live ? f.x : 0.0, q.live ? f.y : 0.0);
+        cplx fc = cmk(0.0, 0.0);
+        if constexpr (AUG)
+            fc = cmul(tq, cfmacj(d, ci, cmk(group_sum(sc[0].x + sc[1].x), group_sum(sc[0].y + sc[1].y))));
+        double n2[2] = {0.0, 0.0};
+        if constexpr (!KEEP) asm volatile("" ::: "memory");   // so that the second reading is one
 #pragma unroll
-        for (int q = 0; q < CPS; ++q) {
-            const int j = i + 1 + seg + q * nseg;
-            const int src = (j == pvt) ? i : j;
-            const bool ok = j < n;
-#pragma unroll
-            for (int k = 0; k < R8; ++k) {
-                const int r = lane8 + 8 * k;
-                a[q][k] = (ok && r < n && r >= i) ? A[r * ld + src] : cmk(0.0, 0.0);
+        for (int k = 0; k < K; ++k) {
+            cplx xk = x[0];
+            if constexpr (KEEP) xk = x[k];
+            else xk = s.vb[lc + LPC * k];
+            if (k == 0) xk = cmk(at ? 0.0 : xk.x, at ? 0.0 : xk.y);
+            q.a[k] = cfma(xk, fa, q.a[k]);
+            if constexpr (AUG) q.c[k] = cfma(xk, fc, q.c[k]);
+            n2[k & 1] = fma(q.a[k].x, q.a[k].x, fma(q.a[k].y, q.a[k].y, n2[k & 1]));
+        }
+        q.n2 = group_sum(n2[0] + n2[1]);
+        // vb is rewritten after the next barrier only, vn1 and the keys before it
+        if (first) {
+            const long long kk = (__double_as_longlong(q.n2) >> 2) + ((long long)q.ex << 51);
+            s.keys[j] = q.live ? (q.n2 == 0.0 ? kOff + 1 : kk) : kOff;
+            s.vn1[j] = q.n2;
+            if (q.live) A[i * ld + j] = cfma(d, fa, ai);   // R(i, j), at the column's first place
+            if constexpr (AUG) {
+                const cplx v = cfma(d, fc, ci);
+                o[i * osr] = cmk(v.x, ocj ? -v.y : v.y);
             }
-            t1[q] = ok ? s.vn1[src] : 0.0;
-            t2[q] = ok ? s.vn2[src] : 0.0;
         }
-        cplx ui = cmk(0.0, 0.0), up = cmk(0.0, 0.0);   // rows < i of columns i and pvt
-        if (tid < i) {
-            ui = A[tid * ld + i];
-            up = A[tid * ld + pvt];
-        }
-        __syncthreads();
-        if (pvt != i && tid < i) {
-            A[tid * ld + i] = up;
-            A[tid * ld + pvt] = ui;
-        }
-        if (seg == 0) {
+        if (own) {
+            if constexpr (!AUG) {
 #pragma unroll
-            for (int k = 0; k < R8; ++k) {
-                const int r = lane8 + 8 * k;
-                if (r < n && r > i) A[r * ld + i] = v[k];
-            }
-            if (lane8 == 0) {
-                A[i * ld + i] = beta;
-                s.tau[i] = tau;
-            }
-        }
-        if (tid == 0 && pvt != i) {
-            const int t = s.piv[pvt];
-            s.piv[pvt] = s.piv[i];
-            s.piv[i] = t;
-        }
-        const cplx ctau = cconj(tau);
-#pragma unroll
-        for (int q = 0; q < CPS; ++q) {
-            const int j = i + 1 + seg + q * nseg;
-            if (j >= n) continue;   // uniform within the segment
-            cplx w = cmk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < R8; ++k) w = cfmacj(v[k], a[q][k], w);
-            w.x = seg8_sum(w.x);
-            w.y = seg8_sum(w.y);
-            const cplx f = cmul(ctau, w);
-            double ai2 = 0.0, rest = 0.0;
-#pragma unroll
-            for (int k = 0; k < R8; ++k) {
-                const int r = lane8 + 8 * k;
-                a[q][k] = csub(a[q][k], cmul(v[k], f));
-                const double m2 = a[q][k].x * a[q][k].x + a[q][k].y * a[q][k].y;
-                if (r == i) ai2 = m2;
-                if (r > i && r < n) rest += m2;
-                if (r < n && r >= i) A[r * ld + j] = a[q][k];
-            }
-            ai2 = seg8_sum(ai2);
-            rest = seg8_sum(rest);
-            // ZLAQP2 norm downdate: temp = max(1 - (|a_ij|/vn1)^2, 0),
-            // recompute if temp (vn1/vn2)^2 <= tol3z, else vn1 *= sqrt(temp);
-            // written as max(vn1^2 - |a_ij|^2, 0) against tol3z vn2^2.
-            const double v1 = t1[q];
-            double nv1 = v1, nv2 = t2[q];
-            if (v1 != 0.0) {
-                bool recompute;
-                if (v1 < 1.0e150 && t2[q] < 1.0e150) {
-                    const double rem = fmax(v1 * v1 - ai2, 0.0);   // = temp * vn1^2
-                    recompute = rem <= tol3z * t2[q] * t2[q];
-                    nv1 = sqrt(rem);
-                } else {
-                    const double tt = sqrt(ai2) / v1;
-                    const double temp = fmax(1.0 - tt * tt, 0.0);
-                    const double qq = v1 / t2[q];
-                    recompute = !(temp * qq * qq > tol3z);
-                    nv1 = v1 * sqrt(temp);
-                }
-                if (recompute) {
-                    if (sumsq_unsafe(rest)) {
-                        __syncwarp(seg8_mask());
-                        nv1 = (i + 1 < n) ? seg8_colnorm(n, ld, A, j, i + 1, lane8) : 0.0;
-                    } else {
-                        nv1 = sqrt(rest);
-                    }
-                    nv2 = nv1;
+                for (int k = 0; k < K; ++k) {
+                    const int r = kb * LPC + lc + LPC * k;
+                    if (r > i && r < n) A[r * ld + j] = q.a[k];   // below the column's R
                 }
             }
-            if (lane8 == 0) {
-                s.vn1[j] = nv1;
-                s.vn2[j] = nv2;
+            if (lc == 0) {
+                const double id2 = zero ? 0.0 : 1.0 / d2;
+                s.piv[i] = j;
+                s.ipiv[j] = i;
+                s.tau[i] = zero ? cmk(0.0, 0.0) : cmk(-d.x * (b * y * y), -d.y * (b * y * y));   // 1 / b = b / |b|^2
+                s.bet[i] = zero ? 0.0 : b;
+                s.vn2[i] = zero ? __longlong_as_double(0x7ff0000000000000LL) : y;   // 1 / |beta|
+                s.scl[i] = cmk(d.x * id2, -d.y * id2);                              // 1 / d
             }
         }
-        __syncthreads();
     }
-    // D = |diag R|, rows of the upper triangle scaled by 1/D
-    for (int i = tid; i < n; i += blockDim.x) {
-        const cplx a = A[i * ld + i];
-        const double d = hypot(a.x, a.y);
-        s.d[i] = d;
-        s.vn1[i] = 1.0 / d;
+#pragma unroll
+    for (int k = 0; k + 1 < K; ++k) {   // the block's rows are done
+        q.a[k] = q.a[k + 1];
+        if constexpr (AUG) q.c[k] = q.c[k + 1];
     }
-    __syncthreads();
-    for (int e = tid; e < n * n; e += blockDim.x) {
-        const int r = div_by(e, dm), c = e - r * n;
-        if (c >= r) {
-            const double x = s.vn1[r];
-            const cplx a = A[r * ld + c];
-            A[r * ld + c] = cmk(a.x * x, a.y * x);
+    q.a[K - 1] = cmk(0.0, 0.0);
+    if constexpr (AUG) q.c[K - 1] = cmk(0.0, 0.0);
+}
+
+template <int LPC, int RPL, bool AUG>
+COLD void qr_columns(int n, int ld, cplx* A, QRScratch s, MatOp in, MatOp out) {
+    n = uni(n);
+    const int tid = threadIdx.x, lc = tid % LPC, j = tid / LPC;
+    const int nthr = (n * LPC + 31) & ~31;
+    if (uni(tid) < nthr) {
+        const bool col = j < n;
+        const int jc = min(j, n - 1);
+        cplx* const o = const_cast<cplx*>(out.p) + jc * out.sc;
+        QrCol<RPL, AUG> q;
+        double m = 0.0;
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+            const int r = lc + LPC * k, rc = min(r, n - 1);
+            const cplx v = A[rc * ld + jc];
+            const bool ok = col && r < n;
+            q.a[k] = cmk(ok ? v.x : 0.0, ok ? v.y : 0.0);
+            m = fmax(m, fmax(fabs(q.a[k].x), fabs(q.a[k].y)));
+            if constexpr (AUG) {
+                cplx w = cmk(r == j ? 1.0 : 0.0, 0.0);
+                if (in.p) {
+                    w = in.p[rc * in.sr + jc * in.sc];
+                    if (in.cj) w.y = -w.y;
+                }
+                q.c[k] = cmk(ok ? w.x : 0.0, ok ? w.y : 0.0);
+            }
+        }
+#pragma unroll
+        for (int d = LPC / 2; d > 0; d >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+        q.ex = scale_exponent(m);
+        const double down = scalbn(1.0, -q.ex);
+        q.n2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+            q.a[k] = cmk(q.a[k].x * down, q.a[k].y * down);
+            q.n2 = fma(q.a[k].x, q.a[k].x, fma(q.a[k].y, q.a[k].y, q.n2));
+        }
+#pragma unroll
+        for (int d = LPC / 2; d > 0; d >>= 1) q.n2 += __shfl_xor_sync(0xffffffffu, q.n2, d);
+        q.live = col;
+        if (lc == 0 && col) {
+            s.keys[j] = q.n2 == 0.0 ? (long long)0x8000000000000001ull : (__double_as_longlong(q.n2) >> 2) + ((long long)q.ex << 51);
+            s.vn1[j] = q.n2;
+            s.ex[j] = q.ex;
+        }
+        // row blocks in three stretches, each with the register rows that its first block needs
+        constexpr int K2 = (2 * RPL + 2) / 3, K3 = (RPL + 2) / 3;
+        const int nb = (n + LPC - 1) / LPC;
+        int kb = 0;
+        for (; nb - kb > K2; ++kb) qr_block<LPC, RPL, RPL, AUG>(n, ld, kb, nthr, A, s, q, o, out.sr, out.cj);
+        for (; nb - kb > K3; ++kb) qr_block<LPC, RPL, K2, AUG>(n, ld, kb, nthr, A, s, q, o, out.sr, out.cj);
+        for (; kb < nb; ++kb) qr_block<LPC, RPL, K3, AUG>(n, ld, kb, nthr, A, s, q, o, out.sr, out.cj);
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        // columns to their places, in pivot order: rows of R divided by |beta| (and scaled back),
+        // the reflector below divided by its leading entry
+        const int i = s.ipiv[jc];
+        const cplx scl = s.scl[i];
+        cplx w[RPL];
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+            const int r = min(lc + LPC * k, n - 1), e = q.ex - s.ex[s.piv[r]];
+            const cplx v = A[r * ld + jc];
+            const double f = s.vn2[r];
+            w[k] = r == i ? cmk(s.bet[i] * f, 0.0) : cmk(scalbn(v.x * f, e), scalbn(v.y * f, e));
+            if (!AUG && r > i) w[k] = cmul(v, scl);
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+            const int r = lc + LPC * k;
+            if (col && r < n && (!AUG || r <= i)) A[r * ld + i] = w[k];
         }
     }
-    for (int k = tid; k < n; k += blockDim.x) s.ipiv[s.piv[k]] = k;
+    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) s.d[i] = scalbn(fabs(s.bet[i]), s.ex[s.piv[i]]);
     __syncthreads();
 }
 

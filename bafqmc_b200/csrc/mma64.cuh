@@ -35,6 +35,8 @@ struct MatOp {
 DEVI MatOp op_n(const cplx* p, int ld) { return MatOp{p, ld, 1, 0}; }
 DEVI MatOp op_c(const cplx* p, int ld) { return MatOp{p, 1, ld, 1}; }   // conjugate transpose
 
+DEVI MatOp op_h(MatOp m) { return MatOp{m.p, m.sc, m.sr, m.cj ? 0 : 1}; }                 // of a view
+
 enum { TRI_NONE = 0, TRI_A_UPPER = 1, TRI_B_LOWER_FROM_C = 2 };
 
 // Pointers of the classes whose matrices are all in shared memory: the products

@@ -18,6 +18,8 @@ namespace bq {
 __constant__ uint32_t c_apow[kMaxPow];   // a^k mod 2^31 for k = 0 .. kMaxPow-1
 
 template <int NMAX> struct Cfg;
+// LPC lanes per column and RPL rows per lane for the pivoted QR, AUG: the second matrix
+// is carried along (both columns fit the registers).
 // MQ tiles per warp, MB at a time, for the complex products and MP for the real ones
 // (mma64.cuh).
 // R8 rows per lane and CPS columns per 8-lane segment for the register-resident
@@ -32,6 +34,8 @@ template <> struct Cfg<16> {
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 1, CPW = 1;
     static constexpr int LEADS = 1, MQ = 1, MB = 1, MP = 2;
+    static constexpr bool AUG = true;
+    static constexpr int LPC = 4, RPL = 4;
 };
 static_assert(16 % 1 == 0 && 16 % 2 == 0, "tile must divide NMAX");
 // N <= 36: two CTAs per SM, all four matrices in shared memory.  (Three CTAs
@@ -43,6 +47,8 @@ template <> struct Cfg<36> {
     static constexpr bool GW = false, GG = false;
     static constexpr int RW = 2, CPW = 1;
     static constexpr int LEADS = 2, MQ = 4, MB = 2, MP = 8;
+    static constexpr bool AUG = true;
+    static constexpr int LPC = 4, RPL = 9;
 };
 // N <= 72: G and U in shared memory, the workspaces in HBM (one CTA per SM)
 template <> struct Cfg<72> {
@@ -51,6 +57,8 @@ template <> struct Cfg<72> {
     static constexpr bool GW = true, GG = false;
     static constexpr int RW = 3, CPW = 1;
     static constexpr int LEADS = 1, MQ = 6, MB = 2, MP = 6;
+    static constexpr bool AUG = false;
+    static constexpr int LPC = 4, RPL = 18;
 };
 // N <= 144 (up to the 12x12 lattice, number-conserving): G, U, both
 // workspaces and a product scratch in HBM after the chain's arena (L2-resident
@@ -65,6 +73,7 @@ template <> struct Cfg<144> {
                          MINB = 1;
     static constexpr bool GW = true, GG = true;
     static constexpr int LEADS = 1;
+    static constexpr bool AUG = false;
     static constexpr int RW = 5, CPW = 2;
 };
 template <int NMAX>
@@ -74,11 +83,17 @@ constexpr bool mma_fits() {   // the CTA's warps hold every tile of a product
     else return C::MQ * (C::THREADS / 32) >= mma_tiles(NMAX) && C::MP * (C::THREADS / 32) >= mma_tiles(NMAX);
 }
 template <int NMAX>
+constexpr bool qr_fits() {
+    using C = Cfg<NMAX>;
+    if constexpr (C::GG) return true;
+    else return C::LPC * C::RPL >= NMAX && ((NMAX * C::LPC + 31) / 32) * 32 <= C::THREADS;
+}
+template <int NMAX>
 constexpr bool cfg_ok() {
     using C = Cfg<NMAX>;
     return NMAX % C::TR == 0 && NMAX % C::TC == 0 && (C::GG || (NMAX / C::TR) * (NMAX / C::TC) <= C::THREADS) &&
            (!C::GG || (C::RW * 32 >= NMAX && C::THREADS >= NMAX && C::GW)) &&
-           mma_fits<NMAX>() && C::MAXE * C::THREADS >= NMAX * NMAX && C::R8 * 8 >= NMAX && C::CPS * (C::THREADS / 8) >= NMAX &&
+           mma_fits<NMAX>() && qr_fits<NMAX>() && C::MAXE * C::THREADS >= NMAX * NMAX && C::R8 * 8 >= NMAX && C::CPS * (C::THREADS / 8) >= NMAX &&
            (C::LD & 1) == 1 && C::LD >= NMAX;
 }
 static_assert(cfg_ok<16>() && cfg_ok<36>() && cfg_ok<72>() && cfg_ok<144>(),
@@ -172,7 +187,8 @@ struct Smem {
         return TcBufs{at<uint32_t>(oTc), at<uint32_t>(oTc + kTcABytes), at<uint32_t>(oTc + 2 * kTcABytes),
                       at<uint32_t>(oTc + 2 * kTcABytes + kTcBBytes), tc_mbar(), *tc_slot()};
     }
-    DEVI QRScratch qr() const { return QRScratch{tau(), piv(), ipiv(), vn1(), vn2(), d(), cbc(), ibc()}; }
+    DEVI QRScratch qr() const { return QRScratch{tau(), piv(), ipiv(), vn1(), vn2(), d(), cbc(), ibc(), col(0), col(1),
+                         reinterpret_cast<long long*>(col(2)), reinterpret_cast<double*>(col(3)), reinterpret_cast<int*>(col(4))}; }
 };
 
 // green_from_M keeps n complex reciprocals in vn1 | vn2
@@ -272,8 +288,16 @@ DEVI void qrp_any(Ctx<NMAX>& x, cplx* A) {
         }
         __syncthreads();
     } else {
-        qrp_inplace<C_::R8, C_::CPS>(x.n, C_::LD, A, x.s.qr());
+        qr_columns<C_::LPC, C_::RPL, false>(x.n, C_::LD, A, x.s.qr(), MatOp{}, MatOp{});
     }
+}
+// The pivoted QR of A; classes with Cfg::AUG also leave Q^H in (the identity if in.p is
+// null) in the view out, the others their reflectors in A for the routines below.
+template <int NMAX>
+DEVI void qr_any(Ctx<NMAX>& x, cplx* A, MatOp in, MatOp out) {
+    using C_ = Cfg<NMAX>;
+    if constexpr (C_::AUG) qr_columns<C_::LPC, C_::RPL, true>(x.n, C_::LD, A, x.s.qr(), in, out);
+    else qrp_any(x, A);
 }
 template <int NMAX>
 DEVI void form_q_any(Ctx<NMAX>& x, const cplx* F, cplx* Q, bool conjT) {
@@ -1268,7 +1292,7 @@ COLD void stab_UR(Ctx<NMAX> x) {
         x.W1()[r * LD + c] = cmul(x.U()[r * LD + c], x.A().DRc[c]);
     }
     __syncthreads();
-    qrp_any(x, x.W1());
+    qr_any(x, x.W1(), MatOp{}, op_c(x.U(), LD));   // U_R <- Q where Q^H is carried along
     for (int i = threadIdx.x; i < n; i += blockDim.x) x.A().DRc[i] = cmk(s.d()[i], 0.0);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int r = div_by(e, dm), c = e - r * n;
@@ -1276,7 +1300,7 @@ COLD void stab_UR(Ctx<NMAX> x) {
     }
     __syncthreads();
     gemm_any(x, x.W2(), op_n(x.W1(), LD), op_n(x.W2(), LD), TRI_A_UPPER);
-    form_q_any(x, x.W1(), x.U(), false);
+    if constexpr (!Cfg<NMAX>::AUG) form_q_any(x, x.W1(), x.U(), false);
     sstore(n, LD, x.A().VRc, x.W2());
     __syncthreads();
 }
@@ -1293,7 +1317,7 @@ COLD void stab_UL(Ctx<NMAX> x) {
         x.W1()[r * LD + c] = cmul(cconj(x.U()[c * LD + r]), x.A().DLc[c]);
     }
     __syncthreads();
-    qrp_any(x, x.W1());
+    qr_any(x, x.W1(), MatOp{}, op_n(x.U(), LD));   // U_L <- Q^H
     for (int i = threadIdx.x; i < n; i += blockDim.x) x.A().DLc[i] = cmk(s.d()[i], 0.0);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int r = div_by(e, dm), c = e - r * n;
@@ -1301,7 +1325,7 @@ COLD void stab_UL(Ctx<NMAX> x) {
     }
     __syncthreads();
     gemm_any(x, x.W2(), op_n(x.W2(), LD), op_c(x.W1(), LD), TRI_B_LOWER_FROM_C);
-    form_q_any(x, x.W1(), x.U(), true);
+    if constexpr (!Cfg<NMAX>::AUG) form_q_any(x, x.W1(), x.U(), true);
     sstore(n, LD, x.A().VLc, x.W2());
     __syncthreads();
 }
@@ -1327,10 +1351,14 @@ COLD void green_from_M(Ctx<NMAX> x, int nt, bool right_local, bool want_logdet) 
     const MatOp URh = right_local ? Uloc : op_c(x.A().URc, n);
     const MatOp ULh = right_local ? op_c(x.A().ULc, n) : Uloc;
     if (nt > L / 2) conj_transpose_any(x, x.W2());
-    qrp_any(x, x.W2());
-    if (nt < L / 2 + 1) {
-        copy_op(n, LD, x.W1(), URh);
-        apply_qh_left_any(x, x.W2(), x.W1());
+    // W1 <- Q^H U_R^H, or U_L^H Q = (Q^H (U_L^H)^H)^H
+    const bool left = nt < L / 2 + 1;
+    qr_any(x, x.W2(), left ? URh : op_h(ULh), left ? op_n(x.W1(), LD) : op_c(x.W1(), LD));
+    if (left) {
+        if constexpr (!Cfg<NMAX>::AUG) {
+            copy_op(n, LD, x.W1(), URh);
+            apply_qh_left_any(x, x.W2(), x.W1());
+        }
         diag_inverse(n, LD, x.W2(), s.d(), rinv, dinv);
         trsm_left_any(x, x.W2(), rinv, dinv, x.W1());
         permute_rows_any(x, x.W1(), false);
@@ -1342,8 +1370,10 @@ COLD void green_from_M(Ctx<NMAX> x, int nt, bool right_local, bool want_logdet) 
             gemm_any(x, x.W2(), Uloc, op_n(x.W1(), LD));
         }
     } else {
-        copy_op(n, LD, x.W1(), ULh);
-        apply_q_right_any(x, x.W2(), x.W1());
+        if constexpr (!Cfg<NMAX>::AUG) {
+            copy_op(n, LD, x.W1(), ULh);
+            apply_q_right_any(x, x.W2(), x.W1());
+        }
         diag_inverse(n, LD, x.W2(), s.d(), rinv, dinv);
         trsm_right_any(x, x.W2(), rinv, dinv, x.W1());
         permute_cols_any(x, x.W1(), false);
