@@ -89,6 +89,24 @@ DEVI double warp_sum(double v) {
     return v;
 }
 
+// dst[k] += sum over the warp of v[k], k < 16, without a barrier: each exchange halves the
+// values a lane still holds (16 shuffles of a double against 80 for 16 separate sums).
+// dst belongs to the warp.
+DEVI void warp_add16(double (&v)[16], double* dst) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 8; h > 0; h >>= 1) {   // partner 2h lanes away
+        const bool up = (lane & (2 * h)) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const double send = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if (!(lane & 1)) dst[lane >> 1] += v[0];
+}
+
 // Block-wide sum of NV values; result valid in every thread. scratch holds
 // NV * (blockDim.x/32) doubles. Contains two __syncthreads.
 template <int NV>

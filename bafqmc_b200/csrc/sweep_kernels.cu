@@ -134,9 +134,11 @@ struct Smem {
     // tensor-core staging (classes with Cfg::TCORE): A hi | A lo | B hi | B lo, then
     // the MMA barrier, the tensor-memory base, the barrier parity and the on flag
     static constexpr bool TCORE = Cfg<NMAX>::TCORE;
-    static constexpr size_t oTc = ((oCnt + 48 + 127) / 128) * 128;
+    static constexpr size_t oMs = oCnt + 48;   // per warp, 16 sums over the sweep's measurements
+    static constexpr size_t oEnd = oMs + 16 * sizeof(double) * (Cfg<NMAX>::THREADS / 32);
+    static constexpr size_t oTc = ((oEnd + 127) / 128) * 128;
     static constexpr size_t oTcBar = oTc + 2 * kTcABytes + 2 * kTcBBytes;
-    static constexpr size_t bytes() { return TCORE ? oTcBar + 32 : oCnt + 48; }
+    static constexpr size_t bytes() { return TCORE ? oTcBar + 32 : oEnd; }
 
     template <class T>
     static DEVI T* at(size_t off) { return reinterpret_cast<T*>(bq_smem + off); }
@@ -176,6 +178,7 @@ struct Smem {
     DEVI uint32_t* seed() const { return at<uint32_t>(oSeed); }
     DEVI int* sxy() const { return at<int>(oSxy); }
     DEVI long long* cnt() const { return at<long long>(oCnt); }
+    DEVI double* msum() const { return at<double>(oMs); }
     DEVI int* strip_warp() const { return at<int>(oCnt + 40); }
     DEVI uint64_t* tc_mbar() const { return at<uint64_t>(oTcBar); }
     DEVI uint32_t* tc_slot() const { return at<uint32_t>(oTcBar + 8); }
@@ -1052,15 +1055,14 @@ COLD void measure(Ctx<NMAX> x) {
     auto& s = x.s;
     const PointDev& P = x.P();
     const int n = x.n, tid = threadIdx.x, lx = P.Lx, ly = P.Ly;
-    const double lq = (double)P.Lq, lq2 = lq * lq;
     const cplx* G = x.G();
     const cplx* ph = s.ph();
     const bool hasK = P.hasK;
     // v: 0 sum Re(t_up), 1 sum |Gc|^2, 2-3 sf_K, 4-5 dw_K, 6-7 sum t_up, 8-9 sum du_i conj(du_j),
     //    10 kinetic, 11 sum Re du, 12 sum |du|^2, 13 sum Re du^2
-    double v[14];
+    double v[16];
 #pragma unroll
-    for (int k = 0; k < 14; ++k) v[k] = 0.0;
+    for (int k = 0; k < 16; ++k) v[k] = 0.0;
     const int* sxy = s.sxy();
     const int T = blockDim.x;
     const uint32_t dm = div_magic(n);
@@ -1110,8 +1112,24 @@ COLD void measure(Ctx<NMAX> x) {
         v[13] += du.x * du.x - du.y * du.y;
         s.obs()[O_SITE + i] += 2.0 * du.x;
     }
-    block_sum<14>(v, s.red());
-    if (tid == 0) {
+    warp_add16(v, s.msum() + 16 * (tid >> 5));
+    if (tid == 0) s.cnt()[4] += 1;
+}
+
+// The sweep's sums over all measurements (every record below is linear in them) into the
+// bin record's scalars.
+template <int NMAX>
+DEVI void measure_finish(Ctx<NMAX>& x) {
+    auto& s = x.s;
+    const PointDev& P = x.P();
+    const double lq = (double)P.Lq, lq2 = lq * lq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v[14];
+        for (int k = 0; k < 14; ++k) {
+            v[k] = 0.0;
+            for (int w = 0; w < Cfg<NMAX>::THREADS / 32; ++w) v[k] += s.msum()[16 * w + k];
+        }
         double* o = s.obs();
         const double onsite = 2.0 * v[13] + v[11];          // sum Re(2 du^2 + du)
         const double dbl = v[12] / lq;                       // doubleOcc sample
@@ -1142,7 +1160,6 @@ COLD void measure(Ctx<NMAX> x) {
         o[O_DEN_DODO + 1] -= v[7] / lq;
         o[O_DEN_UPDO] += v[8] / lq;
         o[O_DEN_UPDO + 1] += v[9] / lq;
-        s.cnt()[4] += 1;
     }
     __syncthreads();
 }
@@ -1162,16 +1179,16 @@ COLD void measure_pair(Ctx<NMAX> x) {
     auto& s = x.s;
     const PointDev& P = x.P();
     const int n = x.n, ns = P.Ns, tid = threadIdx.x, lx = P.Lx, ly = P.Ly;
-    const double lq = (double)P.Lq, lq2 = lq * lq, dns = (double)ns;
+    const double lq2 = (double)P.Lq * (double)P.Lq;
     const cplx* G = x.G();
     const cplx* ph = s.ph();
     const bool hasK = P.hasK;
     // v: 0-1 sum Dbb, 2-3 sum Dbc, 4 sum |D_ij|^2, 5-6 sf_K, 7-8 dw_K, 9 kinetic bonds,
     //    10 sum Re n_b, 11 sum Re Dbc(i,i), 12 sum Re n_b^2, 13 sum Re Dbb(i,i),
-    //    14 sum Re(C_ii - B_ii), 15-16 tr B, 17-18 tr C
-    double v[19];
+    //    14 sum Re(C_ii - B_ii)
+    double v[16], tr[4] = {0.0, 0.0, 0.0, 0.0};   // tr: traces of B and C, warp 0
 #pragma unroll
-    for (int k = 0; k < 19; ++k) v[k] = 0.0;
+    for (int k = 0; k < 16; ++k) v[k] = 0.0;
     const int* sxy = s.sxy();
     const int T = blockDim.x;
     const uint32_t dm = div_magic(ns);
@@ -1220,14 +1237,40 @@ COLD void measure_pair(Ctx<NMAX> x) {
         v[12] += nb.x * nb.x - nb.y * nb.y;
         v[13] += dbb.x;
         v[14] += C.x - B.x;
-        v[15] += B.x;
-        v[16] += B.y;
-        v[17] += C.x;
-        v[18] += C.y;
         s.obs()[O_SITE + i] += 2.0 * nb.x;
     }
-    block_sum<19>(v, s.red());
-    if (tid == 0) {
+    // psf_Gamma takes the product of this slice's traces: warp 0 forms them
+    if (tid < 32) {
+        for (int i = tid; i < ns; i += 32) {
+            const cplx B = G[i * LD + ns + i], C = G[(ns + i) * LD + i];
+            tr[0] += B.x;
+            tr[1] += B.y;
+            tr[2] += C.x;
+            tr[3] += C.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tr[k] = warp_sum(tr[k]);
+        if (tid == 0) {   // (-conj(tr C tr B) + sum |D_ij|^2) / Lq^2, the sum at the end of the sweep
+            s.obs()[O_PSF_GAMMA] -= (tr[2] * tr[0] - tr[3] * tr[1]) / lq2;
+            s.obs()[O_PSF_GAMMA + 1] += (tr[2] * tr[1] + tr[3] * tr[0]) / lq2;
+            s.cnt()[4] += 1;
+        }
+    }
+    warp_add16(v, s.msum() + 16 * (tid >> 5));
+}
+
+template <int NMAX>
+DEVI void measure_pair_finish(Ctx<NMAX>& x) {
+    auto& s = x.s;
+    const PointDev& P = x.P();
+    const double lq = (double)P.Lq, lq2 = lq * lq, dns = (double)P.Ns;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v[15];
+        for (int k = 0; k < 15; ++k) {
+            v[k] = 0.0;
+            for (int w = 0; w < Cfg<NMAX>::THREADS / 32; ++w) v[k] += s.msum()[16 * w + k];
+        }
         double* o = s.obs();
         const double dens = 2.0 * v[10] / dns;
         const double dbl = v[11] / dns;
@@ -1237,8 +1280,6 @@ COLD void measure_pair(Ctx<NMAX> x) {
         const double epair = P.Delta * pair;
         const double chem = -P.mu * dens;
         const double energy = kin + inter + epair;
-        // tr C tr B; psf_Gamma = (-conj(trC trB) + sum |D_ij|^2) / Lq^2
-        const double tcb_re = v[17] * v[15] - v[18] * v[16], tcb_im = v[17] * v[16] + v[18] * v[15];
         o[O_DENSITY_UP] += v[10] / dns;
         o[O_DENSITY_DO] += v[10] / dns;
         o[O_DENSITY] += dens;
@@ -1263,15 +1304,13 @@ COLD void measure_pair(Ctx<NMAX> x) {
         o[O_SF_K + 1] += v[6] / lq2;
         o[O_DW_K] += v[7] / lq2;
         o[O_DW_K + 1] += v[8] / lq2;
-        o[O_PSF_GAMMA] += (v[4] - tcb_re) / lq2;
-        o[O_PSF_GAMMA + 1] += tcb_im / lq2;
+        o[O_PSF_GAMMA] += v[4] / lq2;
         o[O_DEN_UPUP] += v[0] / lq;
         o[O_DEN_UPUP + 1] += v[1] / lq;
         o[O_DEN_DODO] += v[0] / lq;
         o[O_DEN_DODO + 1] -= v[1] / lq;
         o[O_DEN_UPDO] += v[2] / lq;
         o[O_DEN_UPDO + 1] += v[3] / lq;
-        s.cnt()[4] += 1;
     }
     __syncthreads();
 }
@@ -1544,6 +1583,7 @@ DEVI bool setup_ctx(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
 template <int NMAX>
 DEVI void load_obs(Ctx<NMAX>& x) {
     for (int k = threadIdx.x; k < kObsScalars + NMAX; k += blockDim.x) x.s.obs()[k] = 0.0;
+    for (int k = threadIdx.x; k < 16 * (Cfg<NMAX>::THREADS / 32); k += blockDim.x) x.s.msum()[k] = 0.0;
 }
 template <int NMAX>
 DEVI void flush_obs(Ctx<NMAX>& x, double* gobs) {
@@ -1636,6 +1676,8 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) sweep_ker
     sstore(n, Cfg<NMAX>::LD, x.A().URc, x.U());
     }
     sstore(n, Cfg<NMAX>::LD, x.A().G, x.G());
+    if constexpr (PAIR) measure_pair_finish(x);
+    else measure_finish(x);
     flush_obs(x, ka.obs + (long)chain * ka.obs_stride);
     if (threadIdx.x == 0) {
         x.sc->seed = *s.seed();
