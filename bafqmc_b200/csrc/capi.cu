@@ -344,8 +344,24 @@ bool class_holds(int cls, int n, int pairing) {
     return cls_pair == pairing;
 }
 
-// Device descriptor of a point whose expP | expM | phase table start at mats.
-PointDev point_dev(const PointHost& ph, const double2* mats) {
+// The real parts of e^{-dtau K} and e^{+dtau K} back to back, rows padded to point_real_ld
+// (the padding zero), for the classes that read them in place.
+size_t real_mats_len(const PointHost& ph) {
+    return bq::class_hbm_work(point_class(ph)) ? 2 * (size_t)ph.N * bq::point_real_ld(ph.N) : 0;
+}
+void fill_real_mats(const PointHost& ph, double* out) {
+    const int ld = bq::point_real_ld(ph.N);
+    std::memset(out, 0, sizeof(double) * real_mats_len(ph));
+    for (int m = 0; m < 2; ++m) {
+        const zmat& e = m == 0 ? ph.expP : ph.expM;
+        for (int i = 0; i < ph.N; ++i)
+            for (int j = 0; j < ph.N; ++j) out[((size_t)m * ph.N + i) * ld + j] = e.a[2 * ((size_t)i * ph.N + j)];
+    }
+}
+
+// Device descriptor of a point whose expP | expM | phase table start at mats and whose
+// fill_real_mats (if any) at reals.
+PointDev point_dev(const PointHost& ph, const double2* mats, const double* reals) {
     PointDev d;
     std::memset(&d, 0, sizeof d);
     const size_t nn = (size_t)ph.N * ph.N;
@@ -374,6 +390,9 @@ PointDev point_dev(const PointHost& ph, const double2* mats) {
     d.expP = mats;
     d.expM = mats + nn;
     d.phaseR = mats + 2 * nn;
+    d.ldr = bq::point_real_ld(ph.N);
+    d.realP = reals;
+    d.realM = reals + (size_t)ph.N * d.ldr;
     return d;
 }
 
@@ -510,25 +529,28 @@ int bafqmc_create_tuned(const bafqmc_point* pts, int npts, const int32_t* chain_
     }
     if ((e = bq::upload_pow_table(apow.data(), bq::kMaxPow)) != cudaSuccess) return bail(e, "upload_pow_table");
     // point matrices: expP, expM (N*N each) and the K phase table (Lq) per point
-    size_t mat_total = 0;
-    std::vector<size_t> mat_off(npts);
+    size_t mat_total = 0, real_total = 0;   // the real matrices (if the class takes them) follow all the others
+    std::vector<size_t> mat_off(npts), real_off(npts);
     for (int i = 0; i < npts; ++i) {
         mat_off[i] = mat_total;
         mat_total += 2 * (size_t)h->pts[i].N * h->pts[i].N + h->pts[i].Lq;
+        real_off[i] = real_total;
+        real_total += real_mats_len(h->pts[i]);
     }
-    std::vector<double> mats(2 * mat_total);
+    std::vector<double> mats(2 * mat_total + real_total);
     for (int i = 0; i < npts; ++i) {
         const PointHost& ph = h->pts[i];
         const size_t nn = (size_t)ph.N * ph.N;
         std::memcpy(&mats[2 * mat_off[i]], ph.expP.a.data(), sizeof(double) * 2 * nn);
         std::memcpy(&mats[2 * (mat_off[i] + nn)], ph.expM.a.data(), sizeof(double) * 2 * nn);
         std::memcpy(&mats[2 * (mat_off[i] + 2 * nn)], ph.phaseR.data(), sizeof(double) * 2 * ph.Lq);
+        if (real_mats_len(ph)) fill_real_mats(ph, &mats[2 * mat_total + real_off[i]]);
     }
-    if ((e = cudaMalloc(&h->d_mats, sizeof(double2) * mat_total)) != cudaSuccess) return bail(e, "cudaMalloc mats");
-    if ((e = cudaMemcpy(h->d_mats, mats.data(), sizeof(double2) * mat_total, cudaMemcpyHostToDevice)) != cudaSuccess)
+    if ((e = cudaMalloc(&h->d_mats, sizeof(double) * mats.size())) != cudaSuccess) return bail(e, "cudaMalloc mats");
+    if ((e = cudaMemcpy(h->d_mats, mats.data(), sizeof(double) * mats.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return bail(e, "upload mats");
     std::vector<PointDev> pd(npts);
-    for (int i = 0; i < npts; ++i) pd[i] = point_dev(h->pts[i], h->d_mats + mat_off[i]);
+    for (int i = 0; i < npts; ++i) pd[i] = point_dev(h->pts[i], h->d_mats + mat_off[i], reinterpret_cast<double*>(h->d_mats + mat_total) + real_off[i]);
     std::vector<ChainDev> cd(nchains);
     for (int c = 0; c < nchains; ++c) {
         cd[c].point = chain_point[c];
@@ -1323,7 +1345,10 @@ extern "C" int bafqmc_sweep_noalloc(const bafqmc_point* pt, int nchains, int32_t
     unsigned char* base = g_noalloc_base[dev];
     // descriptors staged on the host, copied into the array in one transfer
     std::vector<unsigned char> stage(o_ob, 0);
-    const PointDev d = point_dev(ph, reinterpret_cast<const double2*>(base + o_mt));
+    // A class that reads the real matrices does not read the complex ones: they take their place (they
+    // are smaller, N >= 37 there), so that the array holds as many chains as without them.
+    const bool real = real_mats_len(ph) > 0;
+    const PointDev d = point_dev(ph, reinterpret_cast<const double2*>(base + o_mt), reinterpret_cast<const double*>(base + o_mt));
     std::memcpy(stage.data() + o_pt, &d, sizeof d);
     ChainDev* cd = reinterpret_cast<ChainDev*>(stage.data() + o_ch);
     int* ix = reinterpret_cast<int*>(stage.data() + o_ix);
@@ -1334,8 +1359,12 @@ extern "C" int bafqmc_sweep_noalloc(const bafqmc_point* pt, int nchains, int32_t
         cd[c].phi_off = (long long)c * ph.p.Ltrot * ph.Lq * 2;
         ix[c] = c;
     }
-    std::memcpy(stage.data() + o_mt, ph.expP.a.data(), sizeof(double2) * nn);
-    std::memcpy(stage.data() + o_mt + sizeof(double2) * nn, ph.expM.a.data(), sizeof(double2) * nn);
+    if (real) {
+        fill_real_mats(ph, reinterpret_cast<double*>(stage.data() + o_mt));
+    } else {
+        std::memcpy(stage.data() + o_mt, ph.expP.a.data(), sizeof(double2) * nn);
+        std::memcpy(stage.data() + o_mt + sizeof(double2) * nn, ph.expM.a.data(), sizeof(double2) * nn);
+    }
     std::memcpy(stage.data() + o_mt + 2 * sizeof(double2) * nn, ph.phaseR.data(), sizeof(double2) * ph.Lq);
     CK(cudaMemcpyAsync(base, stage.data(), o_ob, cudaMemcpyHostToDevice, st));
     // the array keeps the previous call's contents: reset what is accumulated

@@ -46,6 +46,8 @@ cudaError_t launch_tau(const KernelArgs& ka, const int* idx, int count, int grid
 // (0 number-conserving, 1 Nambu), and class 6: number-conserving N <= 144
 constexpr int kNumClasses = 7;
 int class_nmax(int cls);
+bool class_hbm_work(int cls);   // the class takes PointDev::realP / realM (its workspaces are in HBM)
+int point_real_ld(int n);       // their row stride in doubles
 size_t smem_bytes(int cls);
 int class_of(int n, int pairing);   // -1 if no class holds n
 long long class_work_elems(int cls); // complex values of HBM workspace per chain

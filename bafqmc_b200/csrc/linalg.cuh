@@ -8,10 +8,9 @@
 // src/common/mymats.f90:20-29): ZGEMM, ZTRMM, ZGEQP3 (unblocked ZLAQP2 path,
 // which LAPACK takes for the matrix sizes here), ZUNGQR, ZUNMQR, ZTRSM,
 // ZLAPMR/ZLAPMT.  They are written for the sweep's sizes (n <= 64): one CTA
-// owns one matrix.  The reflector and triangular-solve sequences run on 8-lane
-// segments that each keep their columns (or rows) of the operand in registers
-// for the whole sequence and reduce with shuffles, so no step needs a block
-// barrier; divisions are replaced by precomputed reciprocals.
+// owns one matrix.  The factorisation and the reflector and triangular-solve
+// sequences keep the columns of their operand in registers and reduce with
+// shuffles; divisions are replaced by precomputed reciprocals.
 #pragma once
 #include "mma64.cuh"
 
@@ -71,59 +70,7 @@ COLD void conj_transpose_inplace(int n, int ld, cplx* A) {
     __syncthreads();
 }
 
-// Segmented (8-lane) reductions used by the column-parallel reflector passes.
-// The mask covers only the calling thread's aligned 8-lane segment, so the
-// segments of one warp may run different trip counts.
-DEVI unsigned seg8_mask() { return 0xffu << (threadIdx.x & 24); }
-DEVI double seg8_sum(double v) {
-    const unsigned m = seg8_mask();
-    v += __shfl_xor_sync(m, v, 4);
-    v += __shfl_xor_sync(m, v, 2);
-    v += __shfl_xor_sync(m, v, 1);
-    return v;
-}
-DEVI double seg8_max(double v) {
-    const unsigned m = seg8_mask();
-    v = fmax(v, __shfl_xor_sync(m, v, 4));
-    v = fmax(v, __shfl_xor_sync(m, v, 2));
-    v = fmax(v, __shfl_xor_sync(m, v, 1));
-    return v;
-}
-
-// Overflow-safe 2-norm of column j, rows [r0, n), computed by one 8-lane segment.
-DEVI double seg8_colnorm(int n, int ld, const cplx* A, int j, int r0, int lane8) {
-    double m = 0.0;
-    for (int r = r0 + lane8; r < n; r += 8) m = fmax(m, fmax(fabs(A[r * ld + j].x), fabs(A[r * ld + j].y)));
-    m = seg8_max(m);
-    if (m == 0.0) return 0.0;
-    double s = 0.0;
-    for (int r = r0 + lane8; r < n; r += 8) {
-        double a = A[r * ld + j].x / m, b = A[r * ld + j].y / m;
-        s += a * a + b * b;
-    }
-    s = seg8_sum(s);
-    return m * sqrt(s);
-}
-
-// Sum of squares of column j, rows r0..n-1, by one 8-lane segment.
-DEVI double seg8_sumsq_col(int n, int ld, const cplx* A, int j, int r0, int lane8) {
-    double ss = 0.0;
-    for (int r = r0 + lane8; r < n; r += 8) {
-        const cplx a = A[r * ld + j];
-        ss = fma(a.x, a.x, fma(a.y, a.y, ss));
-    }
-    return seg8_sum(ss);
-}
-
 DEVI bool sumsq_unsafe(double ss) { return !(ss <= 1.0e300) || (ss != 0.0 && ss < 1.0e-290); }
-
-// 2-norm of column j rows r0..n-1 (one segment); scaled only when the plain sum
-// of squares would over- or underflow.
-DEVI double seg8_norm(int n, int ld, const cplx* A, int j, int r0, int lane8) {
-    const double ss = seg8_sumsq_col(n, ld, A, j, r0, lane8);
-    if (!sumsq_unsafe(ss)) return sqrt(ss);
-    return seg8_colnorm(n, ld, A, j, r0, lane8);
-}
 
 // Shared scratch for the factorisations (lives in shared memory, size ~ 6n).
 struct QRScratch {
@@ -155,7 +102,7 @@ DEVI int scale_exponent(double m) {
 // AUG: also out <- Q^H in for the n x n view `in` (the identity if in.p is null), carried
 // along with the columns of A, so that no pass over the reflectors follows; A's strict
 // lower triangle is then not written.  Otherwise A holds the Householder vectors (unit
-// leading entry implicit) below R, and s.tau their factors, for form_q and apply_*.
+// leading entry implicit) below R, and s.tau their factors, for seq_apply.
 //
 // LPC lanes own a column for the whole factorisation, RPL of its rows each in registers
 // (RPL * LPC >= n), with the same lanes for a column of `in`; pivoting is by bookkeeping,
@@ -386,134 +333,143 @@ COLD void qr_columns(int n, int ld, cplx* A, QRScratch s, MatOp in, MatOp out) {
     __syncthreads();
 }
 
-// C <- Q^H C (ZUNMQR 'L','C'): each segment holds its columns in registers.
-template <int R8, int CPS>
-COLD void apply_qh_left(int n, int ld, const cplx* F, const cplx* tau, cplx* C) {
-    const int tid = threadIdx.x, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    cplx c[CPS][R8];
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            c[q][k] = (j < n && r < n) ? C[r * ld + j] : cmk(0.0, 0.0);
-        }
-    for (int i = 0; i < n; ++i) {
-        const cplx ct = cconj(tau[i]);
-        cplx v[R8];
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = lane8 + 8 * k;
-            v[k] = (r == i) ? cmk(1.0, 0.0) : ((r > i && r < n) ? F[r * ld + i] : cmk(0.0, 0.0));
-        }
-#pragma unroll
-        for (int q = 0; q < CPS; ++q) {
-            cplx w = cmk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < R8; ++k) w = cfmacj(v[k], c[q][k], w);
-            w.x = seg8_sum(w.x);
-            w.y = seg8_sum(w.y);
-            const cplx f = cmul(ct, w);
-#pragma unroll
-            for (int k = 0; k < R8; ++k) c[q][k] = csub(c[q][k], cmul(v[k], f));
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            if (j < n && r < n) C[r * ld + j] = c[q][k];
-        }
-    __syncthreads();
+// The reflector and triangular-solve sequences.  Eight lanes own a column of the operand, RPL of
+// its rows each in registers (RPL * 8 >= n) for CPT columns at once, and walk it block by block of
+// eight steps; a block's columns of F are staged in shared memory (vs: 8 x vld) by the whole CTA
+// with their zeros (and the reflector's unit entry) in place, while the next block's are on their
+// way in registers, so that no step waits for L2 or masks a row.  Rows that are done leave the
+// registers a block at a time, the step count of a block growing or shrinking in three stretches.
+// Bound: the FP64 issue of the updates.  The versions before read F from global memory step by
+// step: 64 columns of a 64 x 64 matrix 250 K (reflectors) and 390 K cycles (solve); 144 x 144
+// 2.3 M and 1.2 M.
+//
+// Element (row r, step i) of what is staged for block b.
+//   SEQ_QH    v_i(r): 0 above i, 1 at i, F(r, i) below;  rows 8b..n-1, steps upwards
+//   SEQ_SOLVE R(r, i) above i, else 0;                   rows 0..8b+7, steps downwards
+enum { SEQ_QH = 0, SEQ_SOLVE = 1 };
+constexpr int kSeqPf = 3;   // prefetched elements per thread
+// A staged column has 8 RPL rows; SEQ_SOLVE also reads (into registers that are never used) the
+// rows before the first that the last stretch reaches.  Odd, so that the eight columns of a row
+// are stored to eight banks.
+template <int RPL> constexpr int kSeqPad = 8 * ((RPL + 2) / 3);
+template <int RPL> constexpr int kSeqLd = 8 * RPL + kSeqPad<RPL> + 1;
+template <int RPL> constexpr int kSeqElems = 8 * kSeqLd<RPL> + kSeqPad<RPL>;
+
+template <int KIND>
+DEVI cplx seq_element(int n, int ld, const cplx* F, int b, int e) {
+    const int kk = e & 7, r = (KIND == SEQ_QH ? 8 * b : 0) + (e >> 3), i = 8 * b + kk;
+    const cplx f = F[min(r, n - 1) * ld + min(i, n - 1)];
+    const bool use = i < n && r < n && (KIND == SEQ_QH ? r > i : r < i);
+    return cmk(use ? f.x : (KIND == SEQ_QH && r == i ? 1.0 : 0.0), use ? f.y : 0.0);
 }
 
-// C <- C Q (ZUNMQR 'R','N'): each segment holds its rows in registers.
-template <int R8, int CPS>
-COLD void apply_q_right(int n, int ld, const cplx* F, const cplx* tau, cplx* C) {
-    const int tid = threadIdx.x, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    cplx c[CPS][R8];   // c[q][k] = C[row seg+q*nseg][col lane8+8k]
+// One block on the K register rows in reach: c[.][k] is row 8b + 8k + lc (SEQ_QH) or
+// 8b - 8k + lc (SEQ_SOLVE); then row block b leaves c[.][0].
+template <int KIND, int RPL, int K, int CPT>
+DEVI void seq_block(int n, int b, const cplx* vs, int vld, const cplx* coef, cplx (&c)[CPT][RPL]) {
+    const int lane = threadIdx.x & 31, lc = lane & 7;
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+        const int kk = KIND == SEQ_QH ? q : 7 - q, i = 8 * b + kk;
+        if (i >= n) continue;
+        const cplx* v = vs + kk * vld + (KIND == SEQ_QH ? lc : 8 * b + lc);   // rows 8k on: + 8k, or - 8k
+        const cplx t = coef[i];
 #pragma unroll
-    for (int q = 0; q < CPS; ++q)
+        for (int m = 0; m < CPT; ++m) {
+            cplx f;
+            if constexpr (KIND == SEQ_QH) {
+                cplx w[2] = {cmk(0.0, 0.0), cmk(0.0, 0.0)};
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = seg + q * nseg, col = lane8 + 8 * k;
-            c[q][k] = (r < n && col < n) ? C[r * ld + col] : cmk(0.0, 0.0);
-        }
-    for (int i = 0; i < n; ++i) {
-        const cplx t = tau[i];
-        cplx v[R8];
+                for (int k = 0; k < K; ++k) w[k & 1] = cfmacj(v[8 * k], c[m][k], w[k & 1]);
+                cplx s = cadd(w[0], w[1]);
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int col = lane8 + 8 * k;
-            v[k] = (col == i) ? cmk(1.0, 0.0) : ((col > i && col < n) ? F[col * ld + i] : cmk(0.0, 0.0));
-        }
+                for (int d = 4; d > 0; d >>= 1) {
+                    s.x += __shfl_xor_sync(0xffffffffu, s.x, d);
+                    s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
+                }
+                f = cmul(cmk(-t.x, t.y), s);   // -conj(tau) v^H c
+            } else {
+                const int src = (lane & 24) + kk;
+                cplx x = cmk(__shfl_sync(0xffffffffu, c[m][0].x, src), __shfl_sync(0xffffffffu, c[m][0].y, src));
+                x = cmul(x, t);
+                c[m][0] = cmk(lc == kk ? x.x : c[m][0].x, lc == kk ? x.y : c[m][0].y);
+                f = cmk(-x.x, -x.y);
+            }
 #pragma unroll
-        for (int q = 0; q < CPS; ++q) {
-            cplx w = cmk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < R8; ++k) w = cfma(c[q][k], v[k], w);
-            w.x = seg8_sum(w.x);
-            w.y = seg8_sum(w.y);
-            const cplx f = cmul(t, w);
-#pragma unroll
-            for (int k = 0; k < R8; ++k) c[q][k] = csub(c[q][k], cmulcj(f, v[k]));
+            for (int k = 0; k < K; ++k) c[m][k] = cfma(v[KIND == SEQ_QH ? 8 * k : -8 * k], f, c[m][k]);
         }
     }
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = seg + q * nseg, col = lane8 + 8 * k;
-            if (r < n && col < n) C[r * ld + col] = c[q][k];
-        }
-    __syncthreads();
 }
 
-// Q = H_0 ... H_{n-1} (ZUNGQR), or Q^H with conjT, written to Q (no alias with F).
-template <int R8, int CPS>
-COLD void form_q(int n, int ld, const cplx* F, const cplx* tau, cplx* Q, bool conjT) {
-    const int tid = threadIdx.x, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    cplx c[CPS][R8];
+// SEQ_QH:    out <- Q^H in, F and coef = tau from qr_columns or qrp_big (the identity if in.p is null)
+// SEQ_SOLVE: out <- P R^{-1} diag(rs) in, coef = 1 / R_ii, row k of the solution to row piv[k]
+// in and out are n x n views (conjugated views serve the products and solves from the right);
+// they may be the same matrix.
+template <int KIND, int RPL, int CPT>
+COLD void seq_apply(int n, int ld, const cplx* F, const cplx* coef, const double* rs, const int* piv, MatOp in, MatOp out,
+                    cplx* buf) {
+    n = uni(n);
+    const int vld = kSeqLd<RPL>;
+    cplx* const vs = buf + kSeqPad<RPL>;
+    const int tid = threadIdx.x, T = blockDim.x, lc = tid & 7, ng = T >> 3;
+    const int nb = (n + 7) >> 3;
+    constexpr int K2 = (2 * RPL + 2) / 3, K3 = (RPL + 2) / 3;
+    cplx* const o = const_cast<cplx*>(out.p);
+    for (int j0 = 0; j0 < n; j0 += ng * CPT) {
+        const int j = j0 + (tid >> 3);
+        cplx c[CPT][RPL];
 #pragma unroll
-    for (int q = 0; q < CPS; ++q)
+        for (int m = 0; m < CPT; ++m)
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            c[q][k] = cmk((r == j) ? 1.0 : 0.0, 0.0);
-        }
-    for (int i = n - 1; i >= 0; --i) {
-        const cplx t = tau[i];
-        cplx v[R8];
+            for (int k = 0; k < RPL; ++k) {
+                const int r = 8 * (KIND == SEQ_QH ? k : nb - 1 - k) + lc, jm = j + m * ng;
+                const int rc = max(min(r, n - 1), 0), jc = min(jm, n - 1);
+                cplx w = cmk(r == jm ? 1.0 : 0.0, 0.0);
+                if (in.p) {
+                    w = in.p[rc * in.sr + jc * in.sc];
+                    if (in.cj) w.y = -w.y;
+                }
+                const double f = KIND == SEQ_SOLVE ? rs[rc] : 1.0;
+                const bool ok = r >= 0 && r < n && jm < n;
+                c[m][k] = cmk(ok ? w.x * f : 0.0, ok ? w.y * f : 0.0);
+            }
+        cplx pf[kSeqPf];
+        int b = KIND == SEQ_QH ? 0 : nb - 1;
+        const int step = KIND == SEQ_QH ? 1 : -1;
 #pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = lane8 + 8 * k;
-            v[k] = (r == i) ? cmk(1.0, 0.0) : ((r > i && r < n) ? F[r * ld + i] : cmk(0.0, 0.0));
-        }
+        for (int q = 0; q < kSeqPf; ++q) pf[q] = seq_element<KIND>(n, ld, F, b, tid + q * T);
+        for (int left = nb; left > 0; --left, b += step) {
+            // SEQ_QH reads all the register rows in reach (zeros past n, as 0 x anything finite is needed)
+            const int rows = KIND == SEQ_QH ? 8 * (left > K2 ? RPL : (left > K3 ? K2 : K3)) : 8 * (b + 1);
+            __syncthreads();   // the staged block is free
 #pragma unroll
-        for (int q = 0; q < CPS; ++q) {
-            const int j = seg + q * nseg;
-            if (j < i) continue;   // columns left of i are untouched by H_i (ZUNG2R), uniform per segment
-            cplx w = cmk(0.0, 0.0);
+            for (int q = 0; q < kSeqPf; ++q) {
+                const int e = tid + q * T;
+                if (e < 8 * rows) vs[(e & 7) * vld + (e >> 3)] = pf[q];
+            }
+            for (int e = tid + kSeqPf * T; e < 8 * rows; e += T) vs[(e & 7) * vld + (e >> 3)] = seq_element<KIND>(n, ld, F, b, e);
+            __syncthreads();
+            const int bn = max(min(b + step, nb - 1), 0);
 #pragma unroll
-            for (int k = 0; k < R8; ++k) w = cfmacj(v[k], c[q][k], w);
-            w.x = seg8_sum(w.x);
-            w.y = seg8_sum(w.y);
-            const cplx f = cmul(t, w);
+            for (int q = 0; q < kSeqPf; ++q) pf[q] = seq_element<KIND>(n, ld, F, bn, tid + q * T);
+            if (uni(j) < n) {   // any column of the warp
+                if (left > K2) seq_block<KIND, RPL, RPL, CPT>(n, b, vs, vld, coef, c);
+                else if (left > K3) seq_block<KIND, RPL, K2, CPT>(n, b, vs, vld, coef, c);
+                else seq_block<KIND, RPL, K3, CPT>(n, b, vs, vld, coef, c);
+            }
 #pragma unroll
-            for (int k = 0; k < R8; ++k) c[q][k] = csub(c[q][k], cmul(v[k], f));
-        }
-    }
+            for (int m = 0; m < CPT; ++m) {
+                const int r = 8 * b + lc, jm = j + m * ng;
+                if (r < n && jm < n) {
+                    const int ro = KIND == SEQ_SOLVE ? piv[r] : r;
+                    o[ro * out.sr + jm * out.sc] = out.cj ? cconj(c[m][0]) : c[m][0];
+                }
 #pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            if (j < n && r < n) {
-                if (conjT) Q[j * ld + r] = cconj(c[q][k]);
-                else Q[r * ld + j] = c[q][k];
+                for (int k = 0; k + 1 < RPL; ++k) c[m][k] = c[m][k + 1];
+                c[m][RPL - 1] = cmk(0.0, 0.0);
             }
         }
+    }
     __syncthreads();
 }
 
@@ -525,170 +481,6 @@ COLD void diag_inverse(int n, int ld, const cplx* F, const double* d, cplx* rinv
         const double id2 = 1.0 / (a.x * a.x + a.y * a.y);
         rinv[i] = cmk(a.x * id2, -a.y * id2);
         dinv[i] = 1.0 / d[i];
-    }
-    __syncthreads();
-}
-
-// C <- R^{-1} diag(rs) C (ZTRSM 'L','U','N','N' after scaling row r of C by
-// rs[r]); rinv from diag_inverse.  Each segment holds its columns in
-// registers; row i's value comes from lane i%8 by shuffle.
-template <int R8, int CPS>
-COLD void trsm_left_upper(int n, int ld, const cplx* F, const cplx* rinv, const double* rs, cplx* C) {
-    const int tid = threadIdx.x, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    const unsigned m = seg8_mask();
-    const int base = tid & 24;
-    cplx c[CPS][R8];
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            if (j < n && r < n) {
-                const cplx x = C[r * ld + j];
-                const double f = rs[r];
-                c[q][k] = cmk(x.x * f, x.y * f);
-            } else {
-                c[q][k] = cmk(0.0, 0.0);
-            }
-        }
-#pragma unroll
-    for (int kk = R8 - 1; kk >= 0; --kk) {
-        for (int l = 7; l >= 0; --l) {
-            const int i = 8 * kk + l;
-            if (i >= n) continue;   // uniform
-            const cplx ri = rinv[i];
-            cplx fcol[R8];
-#pragma unroll
-            for (int k = 0; k < R8; ++k) {
-                const int r = lane8 + 8 * k;
-                fcol[k] = (r < i) ? F[r * ld + i] : cmk(0.0, 0.0);
-            }
-#pragma unroll
-            for (int q = 0; q < CPS; ++q) {
-                cplx x;
-                x.x = __shfl_sync(m, c[q][kk].x, base + l);
-                x.y = __shfl_sync(m, c[q][kk].y, base + l);
-                x = cmul(x, ri);
-                if (lane8 == l) c[q][kk] = x;
-#pragma unroll
-                for (int k = 0; k < R8; ++k) c[q][k] = csub(c[q][k], cmul(fcol[k], x));   // fcol = 0 for rows >= i
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int j = seg + q * nseg, r = lane8 + 8 * k;
-            if (j < n && r < n) C[r * ld + j] = c[q][k];
-        }
-    __syncthreads();
-}
-
-// C <- C diag(cs) R^{-H} (ZTRSM 'R','U','C','N' after scaling column c of C by
-// cs[c]): X R^H = C diag(cs) solved for columns n-1..0.  Each segment holds
-// its rows in registers; column c's value comes from lane c%8.
-template <int R8, int CPS>
-COLD void trsm_right_upperH(int n, int ld, const cplx* F, const cplx* rinv, const double* cs, cplx* C) {
-    const int tid = threadIdx.x, lane8 = tid & 7, seg = tid >> 3, nseg = blockDim.x >> 3;
-    const unsigned m = seg8_mask();
-    const int base = tid & 24;
-    cplx c[CPS][R8];   // c[q][k] = C[row seg+q*nseg][col lane8+8k]
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = seg + q * nseg, col = lane8 + 8 * k;
-            if (r < n && col < n) {
-                const cplx x = C[r * ld + col];
-                const double f = cs[col];
-                c[q][k] = cmk(x.x * f, x.y * f);
-            } else {
-                c[q][k] = cmk(0.0, 0.0);
-            }
-        }
-#pragma unroll
-    for (int kk = R8 - 1; kk >= 0; --kk) {
-        for (int l = 7; l >= 0; --l) {
-            const int cc = 8 * kk + l;
-            if (cc >= n) continue;
-            const cplx ri = cconj(rinv[cc]);   // 1 / conj(R_cc)
-            cplx frow[R8];                      // R[k][cc] for k < cc
-#pragma unroll
-            for (int k = 0; k < R8; ++k) {
-                const int col = lane8 + 8 * k;
-                frow[k] = (col < cc) ? F[col * ld + cc] : cmk(0.0, 0.0);
-            }
-#pragma unroll
-            for (int q = 0; q < CPS; ++q) {
-                cplx x;
-                x.x = __shfl_sync(m, c[q][kk].x, base + l);
-                x.y = __shfl_sync(m, c[q][kk].y, base + l);
-                x = cmul(x, ri);
-                if (lane8 == l) c[q][kk] = x;
-#pragma unroll
-                for (int k = 0; k < R8; ++k) c[q][k] = csub(c[q][k], cmulcj(x, frow[k]));
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < CPS; ++q)
-#pragma unroll
-        for (int k = 0; k < R8; ++k) {
-            const int r = seg + q * nseg, col = lane8 + 8 * k;
-            if (r < n && col < n) C[r * ld + col] = c[q][k];
-        }
-    __syncthreads();
-}
-
-// Row permutation in place.  forward: out[k][:] = in[piv[k]][:] (ZLAPMR .true.,
-// i.e. P^T X); backward: out[piv[k]][:] = in[k][:] (ZLAPMR .false., i.e. P X).
-template <int MAXE>
-COLD void permute_rows(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward) {
-    const uint32_t dm = div_magic(n);
-    cplx v[MAXE];
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = threadIdx.x + k * blockDim.x;
-        if (e < n * n) {
-            const int r = div_by(e, dm), c = e - r * n;
-            v[k] = C[(forward ? piv[r] : ipiv[r]) * ld + c];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = threadIdx.x + k * blockDim.x;
-        if (e < n * n) {
-            const int r = div_by(e, dm), c = e - r * n;
-            C[r * ld + c] = v[k];
-        }
-    }
-    __syncthreads();
-}
-
-// Column permutation in place.  forward: out[:, k] = in[:, piv[k]] (ZLAPMT
-// .true., X P); backward: out[:, piv[k]] = in[:, k] (ZLAPMT .false., X P^T).
-template <int MAXE>
-COLD void permute_cols(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward) {
-    const uint32_t dm = div_magic(n);
-    cplx v[MAXE];
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = threadIdx.x + k * blockDim.x;
-        if (e < n * n) {
-            const int r = div_by(e, dm), c = e - r * n;
-            v[k] = C[r * ld + (forward ? piv[c] : ipiv[c])];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < MAXE; ++k) {
-        const int e = threadIdx.x + k * blockDim.x;
-        if (e < n * n) {
-            const int r = div_by(e, dm), c = e - r * n;
-            C[r * ld + c] = v[k];
-        }
     }
     __syncthreads();
 }

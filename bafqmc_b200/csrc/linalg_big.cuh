@@ -51,156 +51,156 @@ DEVI double warp_norm(int n, int ld, const cplx* A, int j, int r0) {
     return warp_colnorm<CM>(n, ld, A, j, r0);
 }
 
-// C = op(A) op(B), C distinct from A and B; tri as in gemm_rs.
-// Work items are a warp's: with B untransposed (B.sc == 1) lanes take 32
-// consecutive columns of C over kGW rows, so each B(k, :) load is one coalesced
-// row segment and each A(r, k) load is the same address in every lane; with A
-// conjugate-transposed (A.sr == 1) lanes take 32 consecutive rows over kGW
-// columns, the mirror image.  The remaining case (A untransposed, B
-// transposed) keeps per-thread TR x TC tiles.  Every element of C takes the
-// same k-ordered cfma sequence in all three forms.
-constexpr int kGW = 9;
-template <int TR, int TC>
-COLD void gemm_big(int n, int ld, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) {
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int nch = (n + 31) >> 5, items = nch * ((n + kGW - 1) / kGW);
-    if (B.sc == 1) {
-        for (int it = threadIdx.x >> 5; it < items; it += nw) {
-            const int c = (it % nch) * 32 + lane, rb = (it / nch) * kGW, cc = min(c, n - 1);
-            cplx acc[kGW];
-#pragma unroll
-            for (int i = 0; i < kGW; ++i) acc[i] = cmk(0.0, 0.0);
-            for (int k = 0; k < n; ++k) {
-                cplx bv = B.at(k, cc);
-                if (tri == TRI_B_LOWER_FROM_C && k < cc) bv = cmk(0.0, 0.0);
-#pragma unroll
-                for (int i = 0; i < kGW; ++i) {
-                    const int r = rb + i;
-                    cplx av = A.at(min(r, n - 1), k);
-                    if (tri == TRI_A_UPPER && k < r) av = cmk(0.0, 0.0);
-                    acc[i] = cfma(av, bv, acc[i]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kGW; ++i)
-                if (c < n && rb + i < n) C[(rb + i) * ld + c] = acc[i];
-        }
-    } else if (A.sr == 1) {
-        for (int it = threadIdx.x >> 5; it < items; it += nw) {
-            const int r = (it % nch) * 32 + lane, cb = (it / nch) * kGW, rr = min(r, n - 1);
-            cplx acc[kGW];
-#pragma unroll
-            for (int j = 0; j < kGW; ++j) acc[j] = cmk(0.0, 0.0);
-            for (int k = 0; k < n; ++k) {
-                cplx av = A.at(rr, k);
-                if (tri == TRI_A_UPPER && k < rr) av = cmk(0.0, 0.0);
-#pragma unroll
-                for (int j = 0; j < kGW; ++j) {
-                    const int c = cb + j;
-                    cplx bv = B.at(k, min(c, n - 1));
-                    if (tri == TRI_B_LOWER_FROM_C && k < c) bv = cmk(0.0, 0.0);
-                    acc[j] = cfma(av, bv, acc[j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kGW; ++j)
-                if (r < n && cb + j < n) C[r * ld + cb + j] = acc[j];
-        }
-    } else {
-        const int ncg = (n + TC - 1) / TC, nrg = (n + TR - 1) / TR;
-        for (int g = threadIdx.x; g < ncg * nrg; g += blockDim.x) {
-            const int r0 = (g / ncg) * TR, c0 = (g % ncg) * TC;
-            cplx acc[TR][TC];
-#pragma unroll
-            for (int i = 0; i < TR; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; ++j) acc[i][j] = cmk(0.0, 0.0);
-            for (int k = 0; k < n; ++k) {
-                cplx a[TR], b[TC];
-#pragma unroll
-                for (int i = 0; i < TR; ++i) {
-                    const int r = r0 + i;
-                    a[i] = (r < n) ? A.at(r, k) : cmk(0.0, 0.0);
-                    if (tri == TRI_A_UPPER && k < r) a[i] = cmk(0.0, 0.0);
-                }
-#pragma unroll
-                for (int j = 0; j < TC; ++j) {
-                    const int c = c0 + j;
-                    b[j] = (c < n) ? B.at(k, c) : cmk(0.0, 0.0);
-                    if (tri == TRI_B_LOWER_FROM_C && k < c) b[j] = cmk(0.0, 0.0);
-                }
-#pragma unroll
-                for (int i = 0; i < TR; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-            }
-#pragma unroll
-            for (int i = 0; i < TR; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; ++j) {
-                    const int r = r0 + i, c = c0 + j;
-                    if (r < n && c < n) C[r * ld + c] = acc[i][j];
-                }
-        }
-    }
-    __syncthreads();
+// C = A B (n x n <= 144, C apart from the operands) on the FP64 tensor pipe, operands in
+// global memory (L2): k is staged in chunks of 16 through shared memory (`stage`, two
+// buffers, cp.async), for column panels of 64.  KIND as in prod_mma: PROD_CC, or one real
+// operand R (leading dimension ldr, even, rows 16-byte aligned) on the left (R X, X = B) or
+// on the right, taken as C^T = R^T X^T (B = X^T): the complex operand, a chain's own, is
+// then read once and R, which the point's chains share, once per panel.  The matrices of 148
+// chains in flight are more than L2 holds.
+// Each operand is staged in the order it is stored in (rows or columns contiguous), with
+// an odd leading dimension in shared memory, and taken with the fragment maps of
+// mma64.cuh.  A warp owns one column tile of a panel and up to nine row tiles, so a step of
+// four k reads 10 fragments for 18 (real) or 36 mma: 38 of 72, or 40 of 144, cycles of
+// shared memory.  tri as there (zeros are filled in when a chunk is staged).
+// The products of the 12x12 lattice are bound by the mma: 93 K cycles for a complex x real
+// one at 64 FMA/clk; per-thread tiles reading L2 took 500 K.
+constexpr int kBigK = 16, kBigCols = 64, kBigRows = 144;
+constexpr int kBigLa = kBigK + 1, kBigLb = kBigCols + 1, kBigLra = kBigK + 4, kBigLrt = kBigRows + 4;
+constexpr size_t kBigABytes = sizeof(cplx) * kBigRows * kBigLa, kBigBBytes = sizeof(cplx) * kBigCols * kBigLa;
+constexpr size_t kBigStage = 2 * (kBigABytes + kBigBBytes);
+
+DEVI void cp16(void* dst, const void* src, int bytes) {   // the rest of the 16 bytes as zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(bytes)
+                 : "memory");
 }
 
-// C = A B with one real operand (RIGHT_REAL: B real), C distinct from A and B.
-template <int TR, int TC, bool RIGHT_REAL>
-COLD void gemm_big_real(int n, int ld, cplx* C, const void* Ap, const void* Bp) {
-    const int ncg = (n + TC - 1) / TC, nrg = (n + TR - 1) / TR;
-    for (int g = threadIdx.x; g < ncg * nrg; g += blockDim.x) {
-        const int r0 = (g / ncg) * TR, c0 = (g % ncg) * TC;
-        int ra[TR], cb[TC];
+// one staged chunk into the accumulators of the warp's CNT row tiles (from rt0) and column tile ct
+template <int KIND, int CNT>
+DEVI void big_chunk(double (&re)[9][2], double (&im)[9][2], const unsigned char* sa, const unsigned char* sb, int rt0, int nrt,
+                    int ct, int ars, int aks, int bcs, int bks, double ca, double cb) {
+    const int lane = threadIdx.x & 31, l4 = lane & 3, l8 = lane >> 2;
+    const cplx* A = reinterpret_cast<const cplx*>(sa);
+    const cplx* B = reinterpret_cast<const cplx*>(sb);
+    const double* Ra = reinterpret_cast<const double*>(sa);
 #pragma unroll
-        for (int i = 0; i < TR; ++i) ra[i] = min(r0 + i, n - 1) * ld;
+    for (int k4 = 0; k4 < kBigK; k4 += 4) {
+        const int k = k4 + l4;
+        cplx b = B[tile_at(ct, l8) * bcs + k * bks];
+        if (KIND == PROD_CC) b.y *= cb;
 #pragma unroll
-        for (int j = 0; j < TC; ++j) cb[j] = min(c0 + j, n - 1);
-        cplx acc[TR][TC];
-#pragma unroll
-        for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) acc[i][j] = cmk(0.0, 0.0);
-        for (int k = 0; k < n; ++k) {
-            if (RIGHT_REAL) {
-                const cplx* A = static_cast<const cplx*>(Ap);
-                const double* B = static_cast<const double*>(Bp);
-                cplx a[TR];
-                double b[TC];
-#pragma unroll
-                for (int i = 0; i < TR; ++i) a[i] = A[ra[i] + k];
-#pragma unroll
-                for (int j = 0; j < TC; ++j) b[j] = B[k * ld + cb[j]];
-#pragma unroll
-                for (int i = 0; i < TR; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC; ++j)
-                        acc[i][j] = cmk(fma(a[i].x, b[j], acc[i][j].x), fma(a[i].y, b[j], acc[i][j].y));
+        for (int i = 0; i < CNT; ++i) {
+            const int rt = min(rt0 + i, nrt - 1);
+            if constexpr (KIND != PROD_CC) {
+                const double ra = KIND == PROD_REAL_L ? Ra[(8 * rt + l8) * kBigLra + k] : Ra[k * kBigLrt + 8 * rt + l8];
+                mma_f64(re[i][0], re[i][1], ra, b.x);
+                mma_f64(im[i][0], im[i][1], ra, b.y);
             } else {
-                const double* A = static_cast<const double*>(Ap);
-                const cplx* B = static_cast<const cplx*>(Bp);
-                double a[TR];
-                cplx b[TC];
-#pragma unroll
-                for (int i = 0; i < TR; ++i) a[i] = A[ra[i] + k];
-#pragma unroll
-                for (int j = 0; j < TC; ++j) b[j] = B[k * ld + cb[j]];
-#pragma unroll
-                for (int i = 0; i < TR; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC; ++j)
-                        acc[i][j] = cmk(fma(a[i], b[j].x, acc[i][j].x), fma(a[i], b[j].y, acc[i][j].y));
+                cplx a = A[tile_at(rt, l8) * ars + k * aks];
+                a.y *= ca;
+                mma_f64(re[i][0], re[i][1], a.x, b.x);
+                mma_f64(im[i][0], im[i][1], a.x, b.y);
+                mma_f64(re[i][0], re[i][1], -a.y, b.y);
+                mma_f64(im[i][0], im[i][1], a.y, b.x);
             }
         }
-#pragma unroll
-        for (int i = 0; i < TR; ++i)
-#pragma unroll
-            for (int j = 0; j < TC; ++j) {
-                const int r = r0 + i, c = c0 + j;
-                if (r < n && c < n) C[r * ld + c] = acc[i][j];
-            }
     }
+}
+
+template <int KIND>
+COLD void gemm_big(int n, int ldc, cplx* C, MatOp A, MatOp B, const double* R, int ldr, int tri, unsigned char* stage) {
+    n = uni(n);
+    tri = uni(tri);
+    const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = warp_index(), nw = T >> 5;
+    const int l4 = lane & 3, l8 = lane >> 2;
+    const int n8 = (n + 7) >> 3, npan = (n8 + 7) >> 3, nk = (n + kBigK - 1) / kBigK, items = npan * nk;
+    const bool arow = A.sc == 1, brow = B.sc == 1;   // stored with k (A) or columns (B) contiguous
+    const int ars = arow ? kBigLa : 1, aks = arow ? 1 : kBigRows + 1;
+    const int bcs = brow ? 1 : kBigLa, bks = brow ? kBigLb : 1;
+    const double ca = A.cj ? -1.0 : 1.0, cb = B.cj ? -1.0 : 1.0;
+    const auto fill = [&](int it) {
+        if (it < items) {
+            const int pan = it / nk, k0 = (it - pan * nk) * kBigK, c0 = pan * kBigCols;
+            unsigned char* da = stage + (it & 1) * (kBigABytes + kBigBBytes);
+            unsigned char* db = da + kBigABytes;
+            if constexpr (KIND == PROD_REAL_L) {
+                for (int e = tid; e < kBigRows * (kBigK / 2); e += T) {
+                    const int r = e / (kBigK / 2), k = k0 + 2 * (e % (kBigK / 2));
+                    const int ok = r < n ? min(max(n - k, 0), 2) : 0;
+                    cp16(da + 8 * (r * kBigLra + k - k0), R + (ok ? r * ldr + k : 0), 8 * ok);
+                }
+            } else if constexpr (KIND == PROD_REAL_R) {   // R^T: rows contiguous
+                for (int e = tid; e < kBigK * (kBigRows / 2); e += T) {
+                    const int kk = e / (kBigRows / 2), r = 2 * (e % (kBigRows / 2)), k = k0 + kk;
+                    const int ok = k < n ? min(max(n - r, 0), 2) : 0;
+                    cp16(da + 8 * (kk * kBigLrt + r), R + (ok ? k * ldr + r : 0), 8 * ok);
+                }
+            } else if (arow) {
+                for (int e = tid; e < kBigRows * kBigK; e += T) {
+                    const int r = e / kBigK, kk = e % kBigK, k = k0 + kk;
+                    const bool ok = r < n && k < n && !(tri == TRI_A_UPPER && k < r);
+                    cp16(da + 16 * (r * kBigLa + kk), A.p + (ok ? r * A.sr + k : 0), ok ? 16 : 0);
+                }
+            } else {
+                for (int e = tid; e < kBigRows * kBigK; e += T) {
+                    const int kk = e / kBigRows, r = e % kBigRows, k = k0 + kk;
+                    const bool ok = r < n && k < n;
+                    cp16(da + 16 * (kk * (kBigRows + 1) + r), A.p + (ok ? r + k * A.sc : 0), ok ? 16 : 0);
+                }
+            }
+            if (brow) {
+                for (int e = tid; e < kBigK * kBigCols; e += T) {
+                    const int kk = e / kBigCols, cc = e % kBigCols, k = k0 + kk, c = c0 + cc;
+                    const bool ok = k < n && c < n;
+                    cp16(db + 16 * (kk * kBigLb + cc), B.p + (ok ? k * B.sr + c : 0), ok ? 16 : 0);
+                }
+            } else {
+                for (int e = tid; e < kBigCols * kBigK; e += T) {
+                    const int cc = e / kBigK, kk = e % kBigK, k = k0 + kk, c = c0 + cc;
+                    const bool ok = k < n && c < n && !(tri == TRI_B_LOWER_FROM_C && k < c);
+                    cp16(db + 16 * (cc * kBigLa + kk), B.p + (ok ? k + c * B.sc : 0), ok ? 16 : 0);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncthreads();   // the staging buffers are free
+    fill(0);
+    double re[9][2], im[9][2];
+    for (int it = 0; it < items; ++it) {
+        const int pan = it / nk, kc = it - pan * nk;
+        const int pc = min(n8 - 8 * pan, 8), rs = nw / pc, rps = (n8 + rs - 1) / rs;
+        const int ct = warp % pc, rg = warp / pc, rt0 = rg * rps;
+        const bool on = rg < rs && rt0 < n8;
+        if (kc == 0) {
+#pragma unroll
+            for (int i = 0; i < 9; ++i) re[i][0] = re[i][1] = im[i][0] = im[i][1] = 0.0;
+        }
+        fill(it + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const unsigned char* sa = stage + (it & 1) * (kBigABytes + kBigBBytes);
+        const unsigned char* sb = sa + kBigABytes;
+        const int nrt = min(n8, rt0 + rps);
+        if (on) {
+            if (rps > 6) big_chunk<KIND, 9>(re, im, sa, sb, rt0, nrt, ct, ars, aks, bcs, bks, ca, cb);
+            else if (rps > 3) big_chunk<KIND, 6>(re, im, sa, sb, rt0, nrt, ct, ars, aks, bcs, bks, ca, cb);
+            else big_chunk<KIND, 3>(re, im, sa, sb, rt0, nrt, ct, ars, aks, bcs, bks, ca, cb);
+        }
+        __syncthreads();   // the chunk's buffer is filled again by the next turn
+        if (kc == nk - 1 && on) {
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                const int rt = rt0 + i;
+                const int r = KIND == PROD_CC ? tile_at(rt, l8) : 8 * rt + l8, c = pan * kBigCols + 8 * ct + l4;
+                const int rs1 = KIND == PROD_REAL_R ? 1 : ldc, cs1 = KIND == PROD_REAL_R ? ldc : 1;   // transposed back
+                if (rt < nrt && r < n && c < n) C[r * rs1 + c * cs1] = cmk(re[i][0], im[i][0]);
+                if (rt < nrt && r < n && c + 4 < n) C[r * rs1 + (c + 4) * cs1] = cmk(re[i][1], im[i][1]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
 
@@ -217,26 +217,6 @@ COLD void copy_mat(int n, int ld, cplx* dst, const cplx* src) {
 COLD void conj_transpose_big(int n, int ld, cplx* A, cplx* S) {
     copy_op(n, ld, S, op_c(A, ld));
     copy_mat(n, ld, A, S);
-}
-
-// Row / column permutations as permute_rows / permute_cols, through S.
-COLD void permute_rows_big(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward, cplx* S) {
-    const uint32_t dm = div_magic(n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = div_by(e, dm), c = e - r * n;
-        S[r * ld + c] = C[(forward ? piv[r] : ipiv[r]) * ld + c];
-    }
-    __syncthreads();
-    copy_mat(n, ld, C, S);
-}
-COLD void permute_cols_big(int n, int ld, cplx* C, const int* piv, const int* ipiv, bool forward, cplx* S) {
-    const uint32_t dm = div_magic(n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = div_by(e, dm), c = e - r * n;
-        S[r * ld + c] = C[r * ld + (forward ? piv[c] : ipiv[c])];
-    }
-    __syncthreads();
-    copy_mat(n, ld, C, S);
 }
 
 // ZGEQP3 (ZLAQP2 recurrence) + QDRP_decompose post-step, as qrp_inplace.
@@ -411,259 +391,4 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
     for (int k = tid; k < n; k += blockDim.x) s.ipiv[s.piv[k]] = k;
     __syncthreads();
 #undef QA
-}
-
-// v[k] = row lane+32k of reflector i (unit at i, zero above), from column i of F.
-// dst <- src stored column-major (dst[c * ld + r] = src[r * ld + c]).  The
-// reflector and triangular-solve routines below read F one column per warp;
-// with FCM they read such a copy, so each warp load is one contiguous segment.
-COLD void copy_col_major(int n, int ld, cplx* dst, const cplx* src) {
-    const uint32_t dm = div_magic(n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int r = div_by(e, dm), c = e - r * n;
-        dst[c * ld + r] = src[r * ld + c];
-    }
-    __syncthreads();
-}
-
-template <int RW, bool FCM = false>
-DEVI void load_reflector_col(int n, int ld, const cplx* F, int i, cplx (&v)[RW]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < RW; ++k) {
-        const int r = lane + 32 * k;
-        v[k] = (r == i) ? cmk(1.0, 0.0) : ((r > i && r < n) ? F[FCM ? i * ld + r : r * ld + i] : cmk(0.0, 0.0));
-    }
-}
-
-// C <- Q^H C (ZUNMQR 'L','C'): columns of C are independent.
-template <int RW, int CPW, bool FCM = false>
-COLD void apply_qh_left_big(int n, int ld, const cplx* F, const cplx* tau, cplx* C) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int j0 = wp * CPW; j0 < n; j0 += nw * CPW) {
-        cplx c[CPW][RW];
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int j = j0 + q, r = lane + 32 * k;
-                c[q][k] = (j < n && r < n) ? C[r * ld + j] : cmk(0.0, 0.0);
-            }
-        for (int i = 0; i < n; ++i) {
-            const cplx ct = cconj(tau[i]);
-            cplx v[RW];
-            load_reflector_col<RW, FCM>(n, ld, F, i, v);
-#pragma unroll
-            for (int q = 0; q < CPW; ++q) {
-                cplx w = cmk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) w = cfmacj(v[k], c[q][k], w);
-                w.x = warp_sum(w.x);
-                w.y = warp_sum(w.y);
-                const cplx f = cmul(ct, w);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) c[q][k] = csub(c[q][k], cmul(v[k], f));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int j = j0 + q, r = lane + 32 * k;
-                if (j < n && r < n) C[r * ld + j] = c[q][k];
-            }
-    }
-    __syncthreads();
-}
-
-// C <- C Q (ZUNMQR 'R','N'): rows of C are independent.
-template <int RW, int CPW, bool FCM = false>
-COLD void apply_q_right_big(int n, int ld, const cplx* F, const cplx* tau, cplx* C) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int r0 = wp * CPW; r0 < n; r0 += nw * CPW) {
-        cplx c[CPW][RW];   // c[q][k] = C[row r0+q][col lane+32k]
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int r = r0 + q, col = lane + 32 * k;
-                c[q][k] = (r < n && col < n) ? C[r * ld + col] : cmk(0.0, 0.0);
-            }
-        for (int i = 0; i < n; ++i) {
-            const cplx t = tau[i];
-            cplx v[RW];
-            load_reflector_col<RW, FCM>(n, ld, F, i, v);
-#pragma unroll
-            for (int q = 0; q < CPW; ++q) {
-                cplx w = cmk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) w = cfma(c[q][k], v[k], w);
-                w.x = warp_sum(w.x);
-                w.y = warp_sum(w.y);
-                const cplx f = cmul(t, w);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) c[q][k] = csub(c[q][k], cmulcj(f, v[k]));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int r = r0 + q, col = lane + 32 * k;
-                if (r < n && col < n) C[r * ld + col] = c[q][k];
-            }
-    }
-    __syncthreads();
-}
-
-// Q = H_0 ... H_{n-1} (ZUNGQR), or Q^H with conjT, into Q (no alias with F).
-// Column j of Q is H_0 ... H_j e_j.
-template <int RW, int CPW, bool FCM = false>
-COLD void form_q_big(int n, int ld, const cplx* F, const cplx* tau, cplx* Q, bool conjT) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int j0 = wp * CPW; j0 < n; j0 += nw * CPW) {
-        cplx c[CPW][RW];
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) c[q][k] = cmk((lane + 32 * k == j0 + q) ? 1.0 : 0.0, 0.0);
-        for (int i = min(j0 + CPW - 1, n - 1); i >= 0; --i) {
-            const cplx t = tau[i];
-            cplx v[RW];
-            load_reflector_col<RW, FCM>(n, ld, F, i, v);
-#pragma unroll
-            for (int q = 0; q < CPW; ++q) {
-                if (j0 + q < i) continue;   // H_i leaves e_j, j < i, unchanged (ZUNG2R); uniform in the warp
-                cplx w = cmk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) w = cfmacj(v[k], c[q][k], w);
-                w.x = warp_sum(w.x);
-                w.y = warp_sum(w.y);
-                const cplx f = cmul(t, w);
-#pragma unroll
-                for (int k = 0; k < RW; ++k) c[q][k] = csub(c[q][k], cmul(v[k], f));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int j = j0 + q, r = lane + 32 * k;
-                if (j < n && r < n) {
-                    if (conjT) Q[j * ld + r] = cconj(c[q][k]);
-                    else Q[r * ld + j] = c[q][k];
-                }
-            }
-    }
-    __syncthreads();
-}
-
-// C <- R^{-1} diag(rs) C (as trsm_left_upper): columns independent; row i's
-// value comes from lane i % 32 by shuffle.
-template <int RW, int CPW, bool FCM = false>
-COLD void trsm_left_upper_big(int n, int ld, const cplx* F, const cplx* rinv, const double* rs, cplx* C) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int j0 = wp * CPW; j0 < n; j0 += nw * CPW) {
-        cplx c[CPW][RW];
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int j = j0 + q, r = lane + 32 * k;
-                if (j < n && r < n) {
-                    const cplx x = C[r * ld + j];
-                    const double f = rs[r];
-                    c[q][k] = cmk(x.x * f, x.y * f);
-                } else {
-                    c[q][k] = cmk(0.0, 0.0);
-                }
-            }
-#pragma unroll
-        for (int kk = RW - 1; kk >= 0; --kk) {
-            for (int l = 31; l >= 0; --l) {
-                const int i = 32 * kk + l;
-                if (i >= n) continue;   // uniform
-                const cplx ri = rinv[i];
-                cplx fcol[RW];
-#pragma unroll
-                for (int k = 0; k < RW; ++k) {
-                    const int r = lane + 32 * k;
-                    fcol[k] = (r < i) ? F[FCM ? i * ld + r : r * ld + i] : cmk(0.0, 0.0);
-                }
-#pragma unroll
-                for (int q = 0; q < CPW; ++q) {
-                    cplx x;
-                    x.x = __shfl_sync(0xffffffffu, c[q][kk].x, l);
-                    x.y = __shfl_sync(0xffffffffu, c[q][kk].y, l);
-                    x = cmul(x, ri);
-                    if (lane == l) c[q][kk] = x;
-#pragma unroll
-                    for (int k = 0; k < RW; ++k) c[q][k] = csub(c[q][k], cmul(fcol[k], x));
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int j = j0 + q, r = lane + 32 * k;
-                if (j < n && r < n) C[r * ld + j] = c[q][k];
-            }
-    }
-    __syncthreads();
-}
-
-// C <- C diag(cs) R^{-H} (as trsm_right_upperH): rows independent; column c's
-// value comes from lane c % 32.
-template <int RW, int CPW, bool FCM = false>
-COLD void trsm_right_upperH_big(int n, int ld, const cplx* F, const cplx* rinv, const double* cs, cplx* C) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int r0 = wp * CPW; r0 < n; r0 += nw * CPW) {
-        cplx c[CPW][RW];   // c[q][k] = C[row r0+q][col lane+32k]
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int r = r0 + q, col = lane + 32 * k;
-                if (r < n && col < n) {
-                    const cplx x = C[r * ld + col];
-                    const double f = cs[col];
-                    c[q][k] = cmk(x.x * f, x.y * f);
-                } else {
-                    c[q][k] = cmk(0.0, 0.0);
-                }
-            }
-#pragma unroll
-        for (int kk = RW - 1; kk >= 0; --kk) {
-            for (int l = 31; l >= 0; --l) {
-                const int cc = 32 * kk + l;
-                if (cc >= n) continue;
-                const cplx ri = cconj(rinv[cc]);
-                cplx frow[RW];
-#pragma unroll
-                for (int k = 0; k < RW; ++k) {
-                    const int col = lane + 32 * k;
-                    frow[k] = (col < cc) ? F[FCM ? cc * ld + col : col * ld + cc] : cmk(0.0, 0.0);
-                }
-#pragma unroll
-                for (int q = 0; q < CPW; ++q) {
-                    cplx x;
-                    x.x = __shfl_sync(0xffffffffu, c[q][kk].x, l);
-                    x.y = __shfl_sync(0xffffffffu, c[q][kk].y, l);
-                    x = cmul(x, ri);
-                    if (lane == l) c[q][kk] = x;
-#pragma unroll
-                    for (int k = 0; k < RW; ++k) c[q][k] = csub(c[q][k], cmulcj(x, frow[k]));
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < CPW; ++q)
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int r = r0 + q, col = lane + 32 * k;
-                if (r < n && col < n) C[r * ld + col] = c[q][k];
-            }
-    }
-    __syncthreads();
 }

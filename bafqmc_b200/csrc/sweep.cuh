@@ -52,6 +52,8 @@ struct PointDev {
     double shiftLoc, U1, U2, RT, mu, Delta;
     const cplx* expP;      // e^{-dtau K}, N*N row-major
     const cplx* expM;      // e^{+dtau K}
+    const double *realP, *realM;   // real parts of expP and expM (classes with workspaces in HBM), rows padded to ldr
+    int ldr, pad_;
     const cplx* phaseR;    // exp(i K.r) for the Lq lattice displacements r (only if hasK)
 };
 

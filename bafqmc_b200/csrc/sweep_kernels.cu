@@ -19,62 +19,55 @@ __constant__ uint32_t c_apow[kMaxPow];   // a^k mod 2^31 for k = 0 .. kMaxPow-1
 
 template <int NMAX> struct Cfg;
 // LPC lanes per column and RPL rows per lane for the pivoted QR, AUG: the second matrix
-// is carried along (both columns fit the registers).
+// is carried along (both columns fit the registers); SR rows per lane and SC columns per
+// eight lanes for the reflector and solve sequences.
 // MQ tiles per warp, MB at a time, for the complex products and MP for the real ones
 // (mma64.cuh).
-// R8 rows per lane and CPS columns per 8-lane segment for the register-resident
-// factorisation routines: R8 >= NMAX/8, CPS >= NMAX/(THREADS/8).
 // LD: leading dimension of the shared-memory matrices, odd so that a column
 // walk over 16-byte elements touches all eight bank groups.  MINB: CTAs per SM for the register
 // budget.  GW: the two workspaces live in HBM (after the chain's arena) and
 // only G and U in shared memory.
 template <> struct Cfg<16> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 128, TR = 1, TC = 2, MAXE = 2, KB = 8, R8 = 2, CPS = 1, LD = 17, MINB = 4;
+    static constexpr int THREADS = 128, MAXE = 2, KB = 8, LD = 17, MINB = 4;
     static constexpr bool GW = false, GG = false;
-    static constexpr int RW = 1, CPW = 1;
     static constexpr int LEADS = 1, MQ = 1, MB = 1, MP = 2;
     static constexpr bool AUG = true;
-    static constexpr int LPC = 4, RPL = 4;
+    static constexpr int LPC = 4, RPL = 4, SR = 2, SC = 1;
 };
-static_assert(16 % 1 == 0 && 16 % 2 == 0, "tile must divide NMAX");
-// N <= 36: two CTAs per SM, all four matrices in shared memory.  (Three CTAs
-// per SM at 192 threads with the workspaces in HBM measured 42% slower: the
-// slice products and wraps slow down more than the third chain adds.)
+// N <= 36: two CTAs per SM, all four matrices in shared memory.
 template <> struct Cfg<36> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 256, TR = 2, TC = 3, MAXE = 6, KB = 8, R8 = 5, CPS = 2, LD = 37, MINB = 2;
+    static constexpr int THREADS = 256, MAXE = 6, KB = 8, LD = 37, MINB = 2;
     static constexpr bool GW = false, GG = false;
-    static constexpr int RW = 2, CPW = 1;
     static constexpr int LEADS = 2, MQ = 4, MB = 2, MP = 8;
     static constexpr bool AUG = true;
-    static constexpr int LPC = 4, RPL = 9;
+    static constexpr int LPC = 4, RPL = 9, SR = 5, SC = 2;
 };
 // N <= 72: G and U in shared memory, the workspaces in HBM (one CTA per SM)
 template <> struct Cfg<72> {
     static constexpr bool TCORE = false;
-    static constexpr int THREADS = 512, TR = 3, TC = 4, MAXE = 11, KB = 8, R8 = 9, CPS = 2, LD = 73, MINB = 1;
+    static constexpr int THREADS = 512, MAXE = 11, KB = 8, LD = 73, MINB = 1;
     static constexpr bool GW = true, GG = false;
-    static constexpr int RW = 3, CPW = 1;
     static constexpr int LEADS = 1, MQ = 6, MB = 2, MP = 6;
     static constexpr bool AUG = false;
-    static constexpr int LPC = 4, RPL = 18;
+    static constexpr int LPC = 4, RPL = 18, SR = 9, SC = 2;
 };
 // N <= 144 (up to the 12x12 lattice, number-conserving): G, U, both
 // workspaces and a product scratch in HBM after the chain's arena (L2-resident
 // while the chain runs), one CTA of 512 threads per SM.  Neither shared memory
-// nor the register file holds these n x n matrices, so products loop over
-// TR x TC tiles out of place and the factorisations use linalg_big.cuh (one
-// warp per column, RW rows per lane, CPW columns at a time).
+// nor the register file holds these n x n matrices, so products stage panels
+// out of place and the QR runs on a column-major copy, one warp per column with RW
+// rows per lane (linalg_big.cuh).
 static_assert(kTcPer * 512 >= 144 * kTcKC, "tensor-core staging: elements per thread must cover a chunk");
 template <> struct Cfg<144> {
     static constexpr bool TCORE = true;   // slice products may run on the tensor cores (tc.cuh)
-    static constexpr int THREADS = 512, TR = 2, TC = 3, MAXE = 41, KB = 8, R8 = 18, CPS = 3, LD = 145,
+    static constexpr int THREADS = 512, MAXE = 41, KB = 8, LD = 145,
                          MINB = 1;
     static constexpr bool GW = true, GG = true;
     static constexpr int LEADS = 1;
     static constexpr bool AUG = false;
-    static constexpr int RW = 5, CPW = 2;
+    static constexpr int RW = 5, SR = 18, SC = 1;
 };
 template <int NMAX>
 constexpr bool mma_fits() {   // the CTA's warps hold every tile of a product
@@ -85,22 +78,18 @@ constexpr bool mma_fits() {   // the CTA's warps hold every tile of a product
 template <int NMAX>
 constexpr bool qr_fits() {
     using C = Cfg<NMAX>;
-    if constexpr (C::GG) return true;
+    if constexpr (C::GG) return C::RW * 32 >= NMAX && C::THREADS >= NMAX && C::GW;
     else return C::LPC * C::RPL >= NMAX && ((NMAX * C::LPC + 31) / 32) * 32 <= C::THREADS;
 }
 template <int NMAX>
 constexpr bool cfg_ok() {
     using C = Cfg<NMAX>;
-    return NMAX % C::TR == 0 && NMAX % C::TC == 0 && (C::GG || (NMAX / C::TR) * (NMAX / C::TC) <= C::THREADS) &&
-           (!C::GG || (C::RW * 32 >= NMAX && C::THREADS >= NMAX && C::GW)) &&
-           mma_fits<NMAX>() && qr_fits<NMAX>() && C::MAXE * C::THREADS >= NMAX * NMAX && C::R8 * 8 >= NMAX && C::CPS * (C::THREADS / 8) >= NMAX &&
+    return mma_fits<NMAX>() && qr_fits<NMAX>() && C::MAXE * C::THREADS >= NMAX * NMAX && C::SR * 8 >= NMAX &&
+           kSeqElems<C::SR> <= 2 * C::KB * (NMAX + 1) &&
            (C::LD & 1) == 1 && C::LD >= NMAX;
 }
 static_assert(cfg_ok<16>() && cfg_ok<36>() && cfg_ok<72>() && cfg_ok<144>(),
               "class tiles and register layouts must cover NMAX");
-static_assert(36 % 2 == 0 && 36 % 3 == 0, "tile must divide NMAX");
-static_assert(Cfg<16>::R8 * 8 >= 16 && Cfg<16>::CPS * (Cfg<16>::THREADS / 8) >= 16, "register layout must cover NMAX");
-static_assert(Cfg<36>::R8 * 8 >= 36 && Cfg<36>::CPS * (Cfg<36>::THREADS / 8) >= 36, "register layout must cover NMAX");
 
 // Dynamic shared memory of the sweep kernels.  Every buffer sits at a
 // compile-time offset, so device code addresses it without holding pointers.
@@ -180,6 +169,7 @@ struct Smem {
     DEVI long long* cnt() const { return at<long long>(oCnt); }
     DEVI double* msum() const { return at<double>(oMs); }
     DEVI int* strip_warp() const { return at<int>(oCnt + 40); }
+    DEVI unsigned char* stage() const { return at<unsigned char>(oTc); }   // of the FP64 products
     DEVI uint64_t* tc_mbar() const { return at<uint64_t>(oTcBar); }
     DEVI uint32_t* tc_slot() const { return at<uint32_t>(oTcBar + 8); }
     DEVI uint32_t* tc_phase() const { return at<uint32_t>(oTcBar + 12); }
@@ -226,6 +216,20 @@ struct Ctx {
         if constexpr (Smem<NMAX>::GW) return wg + NMAX * Cfg<NMAX>::LD;
         else return s.W2();
     }
+    // e^{-dtau K} and e^{+dtau K}, real, with leading dimension ldr: in the workspaces, or where
+    // those are in HBM the point's own copy, which every chain of the point shares in L2
+    DEVI int ldr() const {
+        if constexpr (Smem<NMAX>::GW) return P().ldr;
+        else return real_ld(NMAX);
+    }
+    DEVI const double* RP() const {
+        if constexpr (Smem<NMAX>::GW) return P().realP;
+        else return reinterpret_cast<const double*>(s.W1());
+    }
+    DEVI const double* RM() const {
+        if constexpr (Smem<NMAX>::GW) return P().realM;
+        else return reinterpret_cast<const double*>(s.W2());
+    }
     DEVI cplx* G() const {
         if constexpr (Smem<NMAX>::GG) return wg + 2 * NMAX * Cfg<NMAX>::LD;
         else return s.G();
@@ -237,8 +241,7 @@ struct Ctx {
     DEVI cplx* S() const { return wg + 4 * NMAX * Cfg<NMAX>::LD; }   // product scratch (HBM-resident classes)
 };
 
-// leading dimension of a class's real e^{-+dtau K}
-template <int NMAX> constexpr int kLdReal = Cfg<NMAX>::GG ? Cfg<NMAX>::LD : real_ld(NMAX);
+static_assert(kBigStage <= 2 * kTcABytes + 2 * kTcBBytes, "the staging buffers of both kinds of product share one region");
 
 // ---------------------------------------------------------------------------
 // Linear algebra per size class: the register-resident 8-lane-segment
@@ -248,26 +251,33 @@ template <int NMAX>
 DEVI void gemm_any(Ctx<NMAX>& x, cplx* C, MatOp A, MatOp B, int tri = TRI_NONE) {
     using C_ = Cfg<NMAX>;
     if constexpr (C_::GG) {
-        gemm_big<C_::TR, C_::TC>(x.n, C_::LD, x.S(), A, B, tri);
-        copy_mat(x.n, C_::LD, C, x.S());
+        const bool alias = C == A.p || C == B.p;   // the product is out of place
+        gemm_big<PROD_CC>(x.n, C_::LD, alias ? x.S() : C, A, B, nullptr, 0, tri, x.s.stage());
+        if (alias) copy_mat(x.n, C_::LD, C, x.S());
     } else {
         gemm_rs<C_::MQ, C_::MB, !C_::GW>(x.n, C_::LD, C, A, B, tri);
     }
 }
-// X <- X R (RIGHT_REAL) or R X, and X2 alike if given (classes with operands in shared memory)
+// Y <- X R (RIGHT_REAL) or R X with Y apart from X (HBM-resident classes)
+template <int NMAX, bool RIGHT_REAL>
+DEVI void gemm_real_out(Ctx<NMAX>& x, cplx* Y, const cplx* X, const double* R) {
+    constexpr int LD = Cfg<NMAX>::LD;
+    gemm_big<RIGHT_REAL ? PROD_REAL_R : PROD_REAL_L>(x.n, LD, Y, MatOp{}, RIGHT_REAL ? MatOp{X, 1, LD, 0} : op_n(X, LD), R,
+                                                     x.ldr(), TRI_NONE, x.s.stage());
+}
+// X <- X R (RIGHT_REAL) or R X, and X2 alike if given
 template <int NMAX, bool RIGHT_REAL>
 DEVI void gemm_real_any(Ctx<NMAX>& x, cplx* X, const double* R, cplx* X2 = nullptr) {
     using C_ = Cfg<NMAX>;
     if constexpr (C_::GG) {
-        if (RIGHT_REAL) gemm_big_real<C_::TR, C_::TC, true>(x.n, C_::LD, x.S(), X, R);
-        else gemm_big_real<C_::TR, C_::TC, false>(x.n, C_::LD, x.S(), R, X);
+        gemm_real_out<NMAX, RIGHT_REAL>(x, x.S(), X, R);
         copy_mat(x.n, C_::LD, X, x.S());
         if (X2) gemm_real_any<NMAX, RIGHT_REAL>(x, X2, R);
     } else {
         // both in one call if the CTA's warps hold both results (they wait in registers)
         const bool two = X2 && 2 * mma_tiles(x.n) > C_::MP * (C_::THREADS / 32);
-        gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, kLdReal<NMAX>, X, R, two ? nullptr : X2);
-        if (two) gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, kLdReal<NMAX>, X2, R, nullptr);
+        gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, x.ldr(), X, R, two ? nullptr : X2);
+        if (two) gemm_smem_real<C_::MP, 2, RIGHT_REAL, !C_::GW>(x.n, C_::LD, x.ldr(), X2, R, nullptr);
     }
 }
 template <int NMAX>
@@ -294,65 +304,25 @@ DEVI void qrp_any(Ctx<NMAX>& x, cplx* A) {
         qr_columns<C_::LPC, C_::RPL, false>(x.n, C_::LD, A, x.s.qr(), MatOp{}, MatOp{});
     }
 }
-// The pivoted QR of A; classes with Cfg::AUG also leave Q^H in (the identity if in.p is
-// null) in the view out, the others their reflectors in A for the routines below.
+// The pivoted QR of A, and out <- Q^H in (the identity if in.p is null): carried along in the
+// classes with Cfg::AUG, from A's reflectors in the others.
 template <int NMAX>
 DEVI void qr_any(Ctx<NMAX>& x, cplx* A, MatOp in, MatOp out) {
     using C_ = Cfg<NMAX>;
-    if constexpr (C_::AUG) qr_columns<C_::LPC, C_::RPL, true>(x.n, C_::LD, A, x.s.qr(), in, out);
-    else qrp_any(x, A);
+    if constexpr (C_::AUG) {
+        qr_columns<C_::LPC, C_::RPL, true>(x.n, C_::LD, A, x.s.qr(), in, out);
+    } else {
+        qrp_any(x, A);
+        seq_apply<SEQ_QH, C_::SR, C_::SC>(x.n, C_::LD, A, x.s.tau(), nullptr, nullptr, in, out, x.s.col(0));
+    }
 }
+// out <- P R^{-1} D^{-1} in for the factorisation in F (ZTRSM after the scaling, ZLAPMR)
 template <int NMAX>
-DEVI void form_q_any(Ctx<NMAX>& x, const cplx* F, cplx* Q, bool conjT) {
+DEVI void solve_any(Ctx<NMAX>& x, const cplx* F, MatOp in, MatOp out) {
     using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) {
-        copy_col_major(x.n, C_::LD, x.S(), F);
-        form_q_big<C_::RW, C_::CPW, true>(x.n, C_::LD, x.S(), x.s.tau(), Q, conjT);
-    } else form_q<C_::R8, C_::CPS>(x.n, C_::LD, F, x.s.tau(), Q, conjT);
-}
-template <int NMAX>
-DEVI void apply_qh_left_any(Ctx<NMAX>& x, const cplx* F, cplx* C) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) {
-        copy_col_major(x.n, C_::LD, x.S(), F);
-        apply_qh_left_big<C_::RW, C_::CPW, true>(x.n, C_::LD, x.S(), x.s.tau(), C);
-    } else apply_qh_left<C_::R8, C_::CPS>(x.n, C_::LD, F, x.s.tau(), C);
-}
-template <int NMAX>
-DEVI void apply_q_right_any(Ctx<NMAX>& x, const cplx* F, cplx* C) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) {
-        copy_col_major(x.n, C_::LD, x.S(), F);
-        apply_q_right_big<C_::RW, C_::CPW, true>(x.n, C_::LD, x.S(), x.s.tau(), C);
-    } else apply_q_right<C_::R8, C_::CPS>(x.n, C_::LD, F, x.s.tau(), C);
-}
-template <int NMAX>
-DEVI void trsm_left_any(Ctx<NMAX>& x, const cplx* F, const cplx* rinv, const double* rs, cplx* C) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) {
-        copy_col_major(x.n, C_::LD, x.S(), F);
-        trsm_left_upper_big<C_::RW, C_::CPW, true>(x.n, C_::LD, x.S(), rinv, rs, C);
-    } else trsm_left_upper<C_::R8, C_::CPS>(x.n, C_::LD, F, rinv, rs, C);
-}
-template <int NMAX>
-DEVI void trsm_right_any(Ctx<NMAX>& x, const cplx* F, const cplx* rinv, const double* cs, cplx* C) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) {
-        copy_col_major(x.n, C_::LD, x.S(), F);
-        trsm_right_upperH_big<C_::RW, C_::CPW, true>(x.n, C_::LD, x.S(), rinv, cs, C);
-    } else trsm_right_upperH<C_::R8, C_::CPS>(x.n, C_::LD, F, rinv, cs, C);
-}
-template <int NMAX>
-DEVI void permute_rows_any(Ctx<NMAX>& x, cplx* C, bool forward) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) permute_rows_big(x.n, C_::LD, C, x.s.piv(), x.s.ipiv(), forward, x.S());
-    else permute_rows<C_::MAXE>(x.n, C_::LD, C, x.s.piv(), x.s.ipiv(), forward);
-}
-template <int NMAX>
-DEVI void permute_cols_any(Ctx<NMAX>& x, cplx* C, bool forward) {
-    using C_ = Cfg<NMAX>;
-    if constexpr (C_::GG) permute_cols_big(x.n, C_::LD, C, x.s.piv(), x.s.ipiv(), forward, x.S());
-    else permute_cols<C_::MAXE>(x.n, C_::LD, C, x.s.piv(), x.s.ipiv(), forward);
+    cplx* rinv = reinterpret_cast<cplx*>(x.s.vn1());   // vn1 | vn2, n complex
+    diag_inverse(x.n, C_::LD, F, x.s.d(), rinv, x.s.u2());
+    seq_apply<SEQ_SOLVE, C_::SR, C_::SC>(x.n, C_::LD, F, rinv, x.s.u2(), x.s.piv(), in, out, x.s.col(0));
 }
 template <int NMAX>
 DEVI void conj_transpose_any(Ctx<NMAX>& x, cplx* A) {
@@ -371,7 +341,7 @@ template <int NMAX, bool RIGHT>
 DEVI void slice_mult(Ctx<NMAX>& x, cplx* X, const double* R) {
     if constexpr (Cfg<NMAX>::TCORE) {
         if (*x.s.tc_on()) {
-            if (tc_product(x.n, Cfg<NMAX>::LD, X, R, RIGHT, x.s.tcb(), x.s.tc_phase(), *x.s.tc_test() != 0,
+            if (tc_product(x.n, Cfg<NMAX>::LD, X, R, x.ldr(), RIGHT, x.s.tcb(), x.s.tc_phase(), *x.s.tc_test() != 0,
                            x.s.tc_pending()))
                 return;
             if (threadIdx.x == 0) {
@@ -472,9 +442,11 @@ DEVI void sload_real(int n, int ld, double* dst, const cplx* src) {
 }
 template <int NMAX>
 DEVI void load_expT(Ctx<NMAX>& x) {
-    sload_real(x.n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
-    sload_real(x.n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W2()), x.P().expM);
-    __syncthreads();
+    if constexpr (!Cfg<NMAX>::GW) {
+        sload_real(x.n, x.ldr(), reinterpret_cast<double*>(x.W1()), x.P().expP);
+        sload_real(x.n, x.ldr(), reinterpret_cast<double*>(x.W2()), x.P().expM);
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1030,13 +1002,18 @@ template <int NMAX, bool LEFT>
 COLD void slice_products(Ctx<NMAX> x) {
     auto& s = x.s;
     const int n = x.n;
-    const double* P = reinterpret_cast<const double*>(x.W1());   // e^{-dtau K}, real
-    const double* M = reinterpret_cast<const double*>(x.W2());   // e^{+dtau K}, real
+    const double *P = x.RP(), *M = x.RM();   // e^{-dtau K}, e^{+dtau K}
     // G and U take the same first factor: one call for both where the products run in place
     if constexpr (Cfg<NMAX>::GG) {
-        slice_mult<NMAX, LEFT>(x, x.G(), P);
-        slice_mult<NMAX, !LEFT>(x, x.G(), M);
-        slice_mult<NMAX, LEFT>(x, x.U(), P);
+        if (*s.tc_on()) {
+            slice_mult<NMAX, LEFT>(x, x.G(), P);
+            slice_mult<NMAX, !LEFT>(x, x.G(), M);
+            slice_mult<NMAX, LEFT>(x, x.U(), P);
+        } else {   // G through the scratch matrix and back: no copy
+            gemm_real_out<NMAX, LEFT>(x, x.S(), x.G(), P);
+            gemm_real_out<NMAX, !LEFT>(x, x.G(), x.S(), M);
+            gemm_real_any<NMAX, LEFT>(x, x.U(), P);
+        }
     } else {
         gemm_real_any<NMAX, LEFT>(x, x.G(), P, x.U());
         gemm_real_any<NMAX, !LEFT>(x, x.G(), M);
@@ -1339,7 +1316,6 @@ COLD void stab_UR(Ctx<NMAX> x) {
     }
     __syncthreads();
     gemm_any(x, x.W2(), op_n(x.W1(), LD), op_n(x.W2(), LD), TRI_A_UPPER);
-    if constexpr (!Cfg<NMAX>::AUG) form_q_any(x, x.W1(), x.U(), false);
     sstore(n, LD, x.A().VRc, x.W2());
     __syncthreads();
 }
@@ -1364,7 +1340,6 @@ COLD void stab_UL(Ctx<NMAX> x) {
     }
     __syncthreads();
     gemm_any(x, x.W2(), op_n(x.W2(), LD), op_c(x.W1(), LD), TRI_B_LOWER_FROM_C);
-    if constexpr (!Cfg<NMAX>::AUG) form_q_any(x, x.W1(), x.U(), true);
     sstore(n, LD, x.A().VLc, x.W2());
     __syncthreads();
 }
@@ -1384,8 +1359,6 @@ COLD void green_from_M(Ctx<NMAX> x, int nt, bool right_local, bool want_logdet) 
     constexpr int LD = Cfg<NMAX>::LD;
     auto& s = x.s;
     const int n = x.n, L = x.P().L;
-    cplx* rinv = reinterpret_cast<cplx*>(s.vn1());   // vn1 | vn2, n complex
-    double* dinv = s.u2();
     const MatOp Uloc = op_c(x.U(), LD);
     const MatOp URh = right_local ? Uloc : op_c(x.A().URc, n);
     const MatOp ULh = right_local ? op_c(x.A().ULc, n) : Uloc;
@@ -1394,13 +1367,7 @@ COLD void green_from_M(Ctx<NMAX> x, int nt, bool right_local, bool want_logdet) 
     const bool left = nt < L / 2 + 1;
     qr_any(x, x.W2(), left ? URh : op_h(ULh), left ? op_n(x.W1(), LD) : op_c(x.W1(), LD));
     if (left) {
-        if constexpr (!Cfg<NMAX>::AUG) {
-            copy_op(n, LD, x.W1(), URh);
-            apply_qh_left_any(x, x.W2(), x.W1());
-        }
-        diag_inverse(n, LD, x.W2(), s.d(), rinv, dinv);
-        trsm_left_any(x, x.W2(), rinv, dinv, x.W1());
-        permute_rows_any(x, x.W1(), false);
+        solve_any(x, x.W2(), op_n(x.W1(), LD), op_n(x.W1(), LD));
         if (right_local) {   // U_L^H from HBM, staged
             sload(n, LD, x.W2(), x.A().ULc);
             __syncthreads();
@@ -1409,13 +1376,7 @@ COLD void green_from_M(Ctx<NMAX> x, int nt, bool right_local, bool want_logdet) 
             gemm_any(x, x.W2(), Uloc, op_n(x.W1(), LD));
         }
     } else {
-        if constexpr (!Cfg<NMAX>::AUG) {
-            copy_op(n, LD, x.W1(), ULh);
-            apply_q_right_any(x, x.W2(), x.W1());
-        }
-        diag_inverse(n, LD, x.W2(), s.d(), rinv, dinv);
-        trsm_right_any(x, x.W2(), rinv, dinv, x.W1());
-        permute_cols_any(x, x.W1(), false);
+        solve_any(x, x.W2(), op_c(x.W1(), LD), op_c(x.W1(), LD));   // from the right: of the conjugate transpose
         if (right_local) {
             gemm_any(x, x.W2(), op_n(x.W1(), LD), Uloc);
         } else {             // U_R^H from HBM, staged
@@ -1720,7 +1681,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
     sstore(n, LD, x.A().URs(0), x.U());
     gcopy(x.A().VRs(0), x.A().VRc, n * n);
     gcopy(x.A().DRs(0), x.A().DRc, n);
-    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
+    if constexpr (!Cfg<NMAX>::GW) sload_real(n, x.ldr(), reinterpret_cast<double*>(x.W1()), x.P().expP);
     __syncthreads();
     const int ns = x.P().Ns;
     for (int nt = 1; nt <= L; ++nt) {
@@ -1739,7 +1700,7 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
             }
             __syncthreads();
         }
-        slice_mult<NMAX, false>(x, x.U(), reinterpret_cast<const double*>(x.W1()));
+        slice_mult<NMAX, false>(x, x.U(), x.RP());
         if (nt % x.P().Nwrap == 0) {
             const int st = nt / x.P().Nwrap;
             stab_UR(x);
@@ -1752,8 +1713,10 @@ __global__ void __launch_bounds__(Cfg<NMAX>::THREADS, Cfg<NMAX>::MINB) pre_kerne
                 scopy(n, LD, x.G(), x.W2());
                 __syncthreads();
             }
-            sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(x.W1()), x.P().expP);
-            __syncthreads();
+            if constexpr (!Cfg<NMAX>::GW) {
+                sload_real(n, x.ldr(), reinterpret_cast<double*>(x.W1()), x.P().expP);
+                __syncthreads();
+            }
         }
     }
     sstore(n, LD, x.A().URc, x.U());
@@ -2052,13 +2015,9 @@ long long tau_region_elems() { return taud::REGION; }
 // Q^H C, R^-1 D^-1, the row permutation back.
 template <int NMAX>
 COLD void tau_solve(Ctx<NMAX>& x, cplx* A, cplx* C) {
-    qrp_any(x, A);
-    apply_qh_left_any(x, A, C);
-    cplx* rinv = reinterpret_cast<cplx*>(x.s.vn1());
-    double* dinv = x.s.u2();
-    diag_inverse(x.n, taud::LD<NMAX>, A, x.s.d(), rinv, dinv);
-    trsm_left_any(x, A, rinv, dinv, C);
-    permute_rows_any(x, C, false);
+    constexpr int LD = taud::LD<NMAX>;
+    qr_any(x, A, op_n(C, LD), op_n(C, LD));
+    solve_any(x, A, op_n(C, LD), op_n(C, LD));
 }
 
 template <int NMAX>
@@ -2205,8 +2164,8 @@ COLD void tau_pass(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
     cplx *sv = slot(x, VEC), *svr = slot(x, VR);
     gcopy(sv, A.DRc, n);
     gcopy(svr, A.VRc, n * n);
-    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(slot(x, EP)), x.P().expP);
-    sload_real(n, kLdReal<NMAX>, reinterpret_cast<double*>(slot(x, EM)), x.P().expM);
+    sload_real(n, x.ldr(), reinterpret_cast<double*>(slot(x, EP)), x.P().expP);
+    sload_real(n, x.ldr(), reinterpret_cast<double*>(slot(x, EM)), x.P().expM);
     sload(n, LD, G, A.G);
     sload(n, LD, x.U(), A.URc);
     __syncthreads();
@@ -2368,6 +2327,8 @@ long long class_work_elems(int cls) {
     return sz == 0 ? w(16, Cfg<16>::LD, Cfg<16>::GW)
                    : (sz == 1 ? w(36, Cfg<36>::LD, Cfg<36>::GW) : w(72, Cfg<72>::LD, Cfg<72>::GW));
 }
+bool class_hbm_work(int cls) { return cls == 6 || cls % 3 == 2; }
+int point_real_ld(int n) { return real_ld(n); }
 size_t smem_bytes(int cls) {
     if (cls == 6) return Smem<144>::bytes();
     const int sz = cls % 3;

@@ -133,7 +133,7 @@ struct TcBufs {
 };
 
 // X <- X R (right) or X <- R X (left) as above, n <= 144, matrices row-major
-// with leading dimension ld.  Called by all threads of the CTA (blockDim.x a
+// with leading dimension ld (R: ldr).  Called by all threads of the CTA (blockDim.x a
 // multiple of 128); returns with the CTA synchronised.  *phase (shared
 // memory) is the parity of the next completion of b.mbar.
 // Returns false if an MMA group did not complete within the poll bound (X is
@@ -142,7 +142,7 @@ struct TcBufs {
 // that the caller waits for it before it releases the tensor memory.
 // wait_test: issue no MMA and poll 1024 times, so that the wait expires with
 // nothing in flight (the test of this give-up path).
-DEVI bool tc_product(int n, int ld, cplx* X, const double* R, bool right, const TcBufs& b, uint32_t* phase,
+DEVI bool tc_product(int n, int ld, cplx* X, const double* R, int ldr, bool right, const TcBufs& b, uint32_t* phase,
                      bool wait_test, uint32_t* pending) {
     cplx* C = X;
     const int tid = threadIdx.x, T = blockDim.x;
@@ -213,7 +213,7 @@ DEVI bool tc_product(int n, int ld, cplx* X, const double* R, bool right, const 
                         kk = e - j * kc;
                     }
                     const int k = k0 + kk;
-                    if (k < n && j < n) v[q] = (right ? R[k * ld + j] : R[j * ld + k]) - (j == k ? 1.0 : 0.0);
+                    if (k < n && j < n) v[q] = (right ? R[k * ldr + j] : R[j * ldr + k]) - (j == k ? 1.0 : 0.0);
                     offs[q] = (kk >> 2) * (kTcNB * 4) + j * 4 + (kk & 3);
                 }
             }
