@@ -339,9 +339,10 @@ COLD void qr_columns(int n, int ld, cplx* A, QRScratch s, MatOp in, MatOp out) {
 // with their zeros (and the reflector's unit entry) in place, while the next block's are on their
 // way in registers, so that no step waits for L2 or masks a row.  Rows that are done leave the
 // registers a block at a time, the step count of a block growing or shrinking in three stretches.
-// Bound: the FP64 issue of the updates.  The versions before read F from global memory step by
-// step: 64 columns of a 64 x 64 matrix 250 K (reflectors) and 390 K cycles (solve); 144 x 144
-// 2.3 M and 1.2 M.
+// Bound: reading the staged block (two 16-byte loads of shared memory per row block and step) and
+// the FP64 issue of the updates.  The versions before read F from global memory step by step:
+// 144 x 144 2.3 M (reflectors) and 1.2 M cycles (solve) against 1.4 M and 0.6 M; wraps of 7x9
+// chains 31.7 -> 24.3 M cycles a sweep.
 //
 // Element (row r, step i) of what is staged for block b.
 //   SEQ_QH    v_i(r): 0 above i, 1 at i, F(r, i) below;  rows 8b..n-1, steps upwards

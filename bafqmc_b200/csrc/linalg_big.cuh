@@ -4,14 +4,11 @@
 // n x n complex matrices a chain works on.  While a chain runs, its region
 // stays in L2.
 //
-// Same operations and conventions as linalg.cuh (ZGEMM/ZTRMM, ZGEQP3 in the
-// ZLAQP2 form with the QDRP_decompose post-step, ZUNGQR, ZUNMQR, ZTRSM,
-// ZLAPMR/ZLAPMT; row-major with leading dimension ld; called by all threads
-// of the block, returning with the block synchronised).  One warp per column
-// (or row) of the operand: lane l holds rows l, l+32, ... (RW >= ceil(n/32) of
-// them) of the warp's current columns, the warp walks its columns in groups
-// of CPW, and reductions are warp shuffles.  Products and permutations are out
-// of place through a scratch matrix S.
+// Same operations and conventions as linalg.cuh (ZGEMM/ZTRMM, ZGEQP3 in the ZLAQP2
+// form with the QDRP_decompose post-step; row-major with leading dimension ld; called
+// by all threads of the block, returning with the block synchronised).  In the QR one
+// warp takes a column: lane l holds rows l, l+32, ... (RW >= ceil(n/32) of them), and
+// reductions are warp shuffles.  Products are out of place through a scratch matrix S.
 #pragma once
 #include "linalg.cuh"
 
@@ -63,8 +60,10 @@ DEVI double warp_norm(int n, int ld, const cplx* A, int j, int r0) {
 // mma64.cuh.  A warp owns one column tile of a panel and up to nine row tiles, so a step of
 // four k reads 10 fragments for 18 (real) or 36 mma: 38 of 72, or 40 of 144, cycles of
 // shared memory.  tri as there (zeros are filled in when a chunk is staged).
-// The products of the 12x12 lattice are bound by the mma: 93 K cycles for a complex x real
-// one at 64 FMA/clk; per-thread tiles reading L2 took 500 K.
+// The mma bound of a complex x real product at n = 144 is 93 K cycles; it takes 160 K by
+// itself and 270 K inside the sweep kernel, where the accumulators share the registers with
+// the callers' state (per-thread tiles reading L2 took 500 K; 256 threads of twice the
+// registers, or panels of 40 columns with six row tiles a warp, were no faster).
 constexpr int kBigK = 16, kBigCols = 64, kBigRows = 144;
 constexpr int kBigLa = kBigK + 1, kBigLb = kBigCols + 1, kBigLra = kBigK + 4, kBigLrt = kBigRows + 4;
 constexpr size_t kBigABytes = sizeof(cplx) * kBigRows * kBigLa, kBigBBytes = sizeof(cplx) * kBigCols * kBigLa;
@@ -219,7 +218,7 @@ COLD void conj_transpose_big(int n, int ld, cplx* A, cplx* S) {
     copy_mat(n, ld, A, S);
 }
 
-// ZGEQP3 (ZLAQP2 recurrence) + QDRP_decompose post-step, as qrp_inplace.
+// ZGEQP3 (ZLAQP2 recurrence) + QDRP_decompose post-step.
 // Per column: every warp finds the pivot and forms the reflector from the
 // pivot column (barrier); the warps update the trailing columns one by one,
 // column pvt from the old column i, with ZLAQP2's norm downdate (barrier);

@@ -490,7 +490,7 @@ DEVI cplx ratio_unit(double ar, double ai, cplx en, cplx eo) {
 //     each accepted term to the submatrix (no barrier per site);
 //  2. block_vectors: the full update vectors of the block from the recorded
 //     coefficients and block values;
-//  3. rank_tiles / rank_rows: G += sum_m X_m Y_m^T on every element.
+//  3. rank_tiles: G += sum_m X_m Y_m^T on every element.
 // Number-conserving (localU.f90:56-71, ZGERU): the rank-1 term of site i is
 // G <- G + coef G(:,i) (e_i - G(i,:))^T.  Nambu (src/pairing/src/localU.f90:33-149
 // on the {b, c^dagger} block): the reference forms the 4x4 P = I + Delta (I -
@@ -752,14 +752,15 @@ DEVI void block_vectors(const Ctx<NMAX>& x, const cplx* G, int n, int k0, int kb
     }
 }
 
-// Step 3 on the FP64 tensor pipe, for the classes whose G is in shared memory: tiles of
+// Step 3 on the FP64 tensor pipe: tiles of
 // 8 x 8 complex elements as in prod_mma, four mma per four slots, NB tiles of a warp in
 // flight; warp w of nw (the lead's scheduler excluded) takes contiguous tiles.  WRAP (the
 // channel's last block): the deferred wrap.  coef() is not read (the lead warp is already
 // writing the next block's).
 template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
 DEVI void rank_tiles(const Ctx<NMAX>& x, cplx* G, int n, int w, int nw, bool flip) {
-    constexpr int LD = Cfg<NMAX>::LD, KB = Cfg<NMAX>::KB, NB = 2;
+    constexpr int LD = Cfg<NMAX>::LD, KB = Cfg<NMAX>::KB;
+    constexpr int NB = Cfg<NMAX>::GG ? 4 : 2;   // G in L2: more loads in flight (12x12 updates 139 -> 137 M cycles)
     const auto& s = x.s;
     n = uni(n);
     w = uni(w);
@@ -815,48 +816,6 @@ DEVI void rank_tiles(const Ctx<NMAX>& x, cplx* G, int n, int w, int nw, bool fli
             if (r[q] < n && c[q] + 4 < n) G[r[q] * LD + c[q] + 4] = g1;
         }
     }
-}
-
-// Step 3 for the classes whose G lives in HBM/L2.  Items are (32-column chunk,
-// PR-row block): a warp's load or store of one row of an item is a coalesced
-// 512-byte segment.  Warp w (of nw, the lead's warp excluded) takes items
-// w, w + nw, ...
-template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
-DEVI void rank_rows(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw, bool flip) {
-    constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD, PR = 9;
-    const auto& s = x.s;
-    const int lane = threadIdx.x & 31;
-    const int nch = (n + 31) >> 5, items = nch * ((n + PR - 1) / PR);
-    for (int it = w; it < items; it += nw) {
-        const int c = (it % nch) * 32 + lane, rb = (it / nch) * PR;
-        if (c >= n) continue;
-        cplx g[PR];
-#pragma unroll
-        for (int a = 0; a < PR; ++a) g[a] = G[min(rb + a, n - 1) * LD + c];
-#pragma unroll
-        for (int m = 0; m < KB; ++m) {
-            if (m >= kb) break;
-            const cplx y = s.row(m)[c];
-            const cplx* cr = s.col(m);
-#pragma unroll
-            for (int a = 0; a < PR; ++a) g[a] = cfma(cr[min(rb + a, n - 1)], y, g[a]);
-        }
-        if constexpr (WRAP) {
-            const cplx fb = wrap_col<NMAX, LEFT, PAIR>(x, c, flip);
-#pragma unroll
-            for (int a = 0; a < PR; ++a)
-                g[a] = cmul(cmul(g[a], wrap_row<NMAX, LEFT, PAIR>(x, min(rb + a, n - 1), flip)), fb);
-        }
-#pragma unroll
-        for (int a = 0; a < PR; ++a)
-            if (rb + a < n) G[(rb + a) * LD + c] = g[a];
-    }
-}
-
-template <int NMAX, bool LEFT, bool PAIR, bool WRAP>
-DEVI void rank_pass(const Ctx<NMAX>& x, cplx* G, int n, int kb, int w, int nw, bool flip) {
-    if constexpr (Cfg<NMAX>::GG) rank_rows<NMAX, LEFT, PAIR, WRAP>(x, G, n, kb, w, nw, flip);
-    else rank_tiles<NMAX, LEFT, PAIR, WRAP>(x, G, n, w, nw, flip);
 }
 
 // Start the copy of a slice's fields (both channels) into shared memory: issued before the
@@ -960,9 +919,9 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
                 if (lead) nacc += c;
             }
         } else if (more) {
-            if (rw >= 0) rank_pass<NMAX, LEFT, PAIR, false>(x, G, n, kb, rw, NRW, flip);
+            if (rw >= 0) rank_tiles<NMAX, LEFT, PAIR, false>(x, G, n, rw, NRW, flip);
         } else if (rw >= 0) {
-            rank_pass<NMAX, LEFT, PAIR, true>(x, G, n, kb, rw, NRW, flip);
+            rank_tiles<NMAX, LEFT, PAIR, true>(x, G, n, rw, NRW, flip);
         }
         __syncthreads();
     }
