@@ -31,7 +31,7 @@ template <> struct Cfg<16> {
     static constexpr bool TCORE = false;
     static constexpr int THREADS = 128, MAXE = 2, KB = 8, LD = 17, MINB = 4;
     static constexpr bool GW = false, GG = false;
-    static constexpr int LEADS = 1, MQ = 1, MB = 1, MP = 2;
+    static constexpr int MQ = 1, MB = 1, MP = 2;
     static constexpr bool AUG = true;
     static constexpr int LPC = 4, RPL = 4, SR = 2, SC = 1;
 };
@@ -40,7 +40,7 @@ template <> struct Cfg<36> {
     static constexpr bool TCORE = false;
     static constexpr int THREADS = 256, MAXE = 6, KB = 8, LD = 37, MINB = 2;
     static constexpr bool GW = false, GG = false;
-    static constexpr int LEADS = 2, MQ = 4, MB = 2, MP = 8;
+    static constexpr int MQ = 4, MB = 2, MP = 8;
     static constexpr bool AUG = true;
     static constexpr int LPC = 4, RPL = 9, SR = 5, SC = 2;
 };
@@ -49,7 +49,7 @@ template <> struct Cfg<72> {
     static constexpr bool TCORE = false;
     static constexpr int THREADS = 512, MAXE = 11, KB = 8, LD = 73, MINB = 1;
     static constexpr bool GW = true, GG = false;
-    static constexpr int LEADS = 1, MQ = 6, MB = 2, MP = 6;
+    static constexpr int MQ = 6, MB = 2, MP = 6;
     static constexpr bool AUG = false;
     static constexpr int LPC = 4, RPL = 18, SR = 9, SC = 2;
 };
@@ -65,7 +65,6 @@ template <> struct Cfg<144> {
     static constexpr int THREADS = 512, MAXE = 41, KB = 8, LD = 145,
                          MINB = 1;
     static constexpr bool GW = true, GG = true;
-    static constexpr int LEADS = 1;
     static constexpr bool AUG = false;
     static constexpr int RW = 5, SR = 18, SC = 1;
 };
@@ -168,7 +167,6 @@ struct Smem {
     DEVI int* sxy() const { return at<int>(oSxy); }
     DEVI long long* cnt() const { return at<long long>(oCnt); }
     DEVI double* msum() const { return at<double>(oMs); }
-    DEVI int* strip_warp() const { return at<int>(oCnt + 40); }
     DEVI unsigned char* stage() const { return at<unsigned char>(oTc); }   // of the FP64 products
     DEVI uint64_t* tc_mbar() const { return at<uint64_t>(oTcBar); }
     DEVI uint32_t* tc_slot() const { return at<uint32_t>(oTcBar + 8); }
@@ -205,7 +203,6 @@ struct Ctx {
     ChainScalars* sc;
     cplx* wg;   // HBM region after the arena: W1, W2 (N > 36), then G, U and a product scratch (N > 72)
     int n;
-    int sw0;    // the local update's deciding warp
     DEVI const PointDev& P() const { return *s.P(); }
     DEVI Arena A() const { return make_arena(abase, n); }
     DEVI cplx* W1() const {
@@ -564,7 +561,7 @@ DEVI cplx shfl_c(cplx v, int src) {
     return cmk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// Step 1, by the lead warp (warp sw0 of the CTA).  Lane l holds the elements
+// Step 1, by the lead warp (warp 0 of the CTA).  Lane l holds the elements
 // (l / 8, l % 8) and (l / 8 + 4, l % 8) of the block's submatrix: the snapshot plus
 // the previous block's kbp terms (to rounding the G that the pass writes there).
 // The decisions run in visiting order, every lane computing the same ratio from the
@@ -835,7 +832,6 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
     constexpr int KB = Cfg<NMAX>::KB, LD = Cfg<NMAX>::LD, W = PAIR ? 2 : 1, SB = KB / W;   // SB sites a block
     auto& s = x.s;
     const int n = uni(x.n), ns = uni(x.P().Ns), tid = threadIdx.x;
-    x.sw0 = uni(x.sw0);
     const double ar = x.P().alpha_re[ch], ai = x.P().alpha_im[ch];
     const double shift = fabs(x.P().shiftLoc);
     const bool flip = PAIR && x.P().flip[ch] != 0;
@@ -882,22 +878,23 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
     }
     __syncthreads();
 
-    // Blocks of SB sites in visiting order.  The lead warp (warp sw0) decides
+    // Blocks of SB sites in visiting order.  The lead warp (warp 0) decides
     // block b + 1 while the other warps run block b's rank pass: it
     // copies block b + 1's submatrix during block b's vector step (G is not
     // written then) and adds block b's terms itself.  The last block's pass applies
     // the channel's deferred wrap.
     constexpr int NT = Cfg<NMAX>::THREADS;
-    const bool lead = tid == 32 * x.sw0;
+    const bool lead = tid == 0;
     const int warp = warp_index();
-    const bool lwarp = warp == x.sw0;
+    const bool lwarp = warp == 0;
     // The lead's chain of dependent FP64 operations waits behind every mma (16 cycles) that
-    // another warp has on its scheduler (warp index modulo 4), so the pass leaves the
-    // schedulers of the leads alone: two of them with two CTAs on the SM, else one.
-    constexpr bool TWO = Cfg<NMAX>::LEADS == 2;
-    const int rel = (warp - x.sw0) & 3;
-    const int rw = TWO ? ((rel & 1) ? warp >> 1 : -1) : (rel ? (warp >> 2) * 3 + rel - 1 : -1);
-    constexpr int NRW = TWO ? NT / 64 : NT / 32 * 3 / 4;
+    // another warp has on its scheduler (warp index modulo 4), so the pass leaves the lead's
+    // scheduler alone.  Every CTA of an SM decides on warp 0: their leads share one scheduler,
+    // which no pass uses.  Leads spread over the schedulers wait for the other CTAs' mma: a 6x6
+    // sweep of two chains an SM 25.7 ms with the pass on two schedulers only, 24.3 on three,
+    // 24.1 here; 4x4 chains, 14 an SM, 20.4 against 18.6 ms.
+    const int rw = (warp & 3) ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;
+    constexpr int NRW = NT / 32 * 3 / 4;
     long long nacc = 0;   // accepted proposals, counted by the lead
     if (lwarp) {
         const int kb = W * min(SB, ns);
@@ -928,7 +925,7 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
     // accepted fields, counters, seed, and the U factor wrap with the final fields
     for (int i = tid; i < ns; i += blockDim.x)
         if (s.accf()[i]) phis[i * 2 + ch] = s.phin()[i];   // the other channel's staged values stay as they are
-    if (tid == 32 * x.sw0) {   // the lead thread: AccCounter%count, kept in shared memory
+    if (lead) {   // AccCounter%count, kept in shared memory
         s.cnt()[ch] += nacc;
         s.cnt()[2 + ch] += ns;
         *s.seed() = lcg_mul(c_apow[2 * ns], s0);
@@ -1475,14 +1472,6 @@ DEVI bool setup_ctx(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
     const ChainDev cd = ka.chains[chain];
     if (threadIdx.x == 0) {
         *x.s.P() = ka.pts[cd.point];
-        // The SM's schedulers take warps by slot modulo 4, so the deciding warps
-        // of two CTAs on one SM would share a scheduler if both used warp 0.  A
-        // CTA whose warp slots start at an odd multiple of 8 decides on warp 2; the
-        // four-warp CTAs, several to an SM, take the warp of their place among four.
-        // Thread 0 decides for the whole CTA.
-        unsigned slot;
-        asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
-        *x.s.strip_warp() = Cfg<NMAX>::THREADS >= 192 ? (((slot >> 3) & 1) ? 2 : 0) : (slot >> 2) & 3;
     }
     __syncthreads();
     x.n = x.P().N;
@@ -1494,7 +1483,6 @@ DEVI bool setup_ctx(Ctx<NMAX>& x, const KernelArgs& ka, int chain) {
     }
     x.abase = ka.arena + cd.arena_off;
     x.wg = x.abase + arena_base(x.n, x.P().Nst);
-    x.sw0 = *x.s.strip_warp();
     x.phi = ka.phi + cd.phi_off;
     x.sc = ka.sc + chain;
     return x.n <= NMAX;
