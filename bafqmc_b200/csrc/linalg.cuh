@@ -5,8 +5,8 @@
 //
 // These restate the LAPACK/BLAS operations the reference sweep calls
 // (src/number_conserving/src/stabilization.f90:41-190 and
-// src/common/mymats.f90:20-29): ZGEMM, ZTRMM, ZGEQP3 (unblocked ZLAQP2 path,
-// which LAPACK takes for the matrix sizes here), ZUNGQR, ZUNMQR, ZTRSM,
+// src/common/mymats.f90:20-29): ZGEMM, ZTRMM, ZGEQP3 (its pivoting, with exact
+// remaining norms in place of ZLAQP2's downdated ones), ZUNGQR, ZUNMQR, ZTRSM,
 // ZLAPMR/ZLAPMT.  They are written for the sweep's sizes (n <= 64): one CTA
 // owns one matrix.  The factorisation and the reflector and triangular-solve
 // sequences keep the columns of their operand in registers and reduce with
@@ -80,8 +80,6 @@ struct QRScratch {
     double* vn1;    // n
     double* vn2;    // n
     double* d;      // n   |R_ii|
-    cplx* bcast;    // 4   broadcast slots
-    int* ibcast;    // 4
     // qr_columns only, in buffers of the local update
     cplx* vb;         // n   the pivot column
     cplx* scl;        // n   1 / d of the reflectors

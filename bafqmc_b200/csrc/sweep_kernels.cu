@@ -109,14 +109,14 @@ struct Smem {
     static constexpr size_t oXb = oRow + BV, oYb = oXb + BB, oSnap = oYb + BB, oFld = oSnap + BB, oDelta = oFld + VC;
     static constexpr size_t oDelta2 = oDelta + VC;
     static constexpr size_t oEao = oDelta2 + VC, oEan = oEao + VC, oEbo = oEan + VC, oEbn = oEbo + VC;
-    static constexpr size_t oPh = oEbn + VC, oCoef = oPh + VC, oCbc = oCoef + 2 * KB * sizeof(cplx);
-    static constexpr size_t oP = oCbc + 4 * sizeof(cplx);
+    static constexpr size_t oPh = oEbn + VC, oCoef = oPh + VC;
+    static constexpr size_t oP = oCoef + 2 * KB * sizeof(cplx);
     static constexpr size_t oRg = oP + ((sizeof(PointDev) + 15) / 16) * 16;
     static constexpr size_t oU2 = oRg + VD, oPhin = oU2 + VD, oVn1 = oPhin + VD, oVn2 = oVn1 + VD, oD = oVn2 + VD;
     static constexpr size_t oRed = oD + VD, oObs = oRed + sizeof(double) * kRed;
     static constexpr size_t oPiv = oObs + sizeof(double) * (kObsScalars + NMAX);
     static constexpr size_t oIpiv = oPiv + sizeof(int) * NMAX, oAccf = oIpiv + sizeof(int) * NMAX;
-    static constexpr size_t oIbc = oAccf + sizeof(int) * NMAX, oSeed = oIbc + 4 * sizeof(int);
+    static constexpr size_t oSeed = oAccf + sizeof(int) * NMAX;
     static constexpr size_t oSxy = oSeed + 16;   // site coordinates x | y << 16
     static constexpr size_t oCnt = oSxy + ((sizeof(int) * NMAX + 15) / 16) * 16;   // nacc[2], nc[2], nobs of the sweep
     // tensor-core staging (classes with Cfg::TCORE): A hi | A lo | B hi | B lo, then
@@ -149,7 +149,6 @@ struct Smem {
     DEVI cplx* ebn() const { return at<cplx>(oEbn); }
     DEVI cplx* ph() const { return at<cplx>(oPh); }
     DEVI cplx* coef() const { return at<cplx>(oCoef); }
-    DEVI cplx* cbc() const { return at<cplx>(oCbc); }
     DEVI PointDev* P() const { return at<PointDev>(oP); }
     DEVI double* rg() const { return at<double>(oRg); }
     DEVI double* u2() const { return at<double>(oU2); }
@@ -162,7 +161,6 @@ struct Smem {
     DEVI int* piv() const { return at<int>(oPiv); }
     DEVI int* ipiv() const { return at<int>(oIpiv); }
     DEVI int* accf() const { return at<int>(oAccf); }
-    DEVI int* ibc() const { return at<int>(oIbc); }
     DEVI uint32_t* seed() const { return at<uint32_t>(oSeed); }
     DEVI int* sxy() const { return at<int>(oSxy); }
     DEVI long long* cnt() const { return at<long long>(oCnt); }
@@ -178,7 +176,7 @@ struct Smem {
         return TcBufs{at<uint32_t>(oTc), at<uint32_t>(oTc + kTcABytes), at<uint32_t>(oTc + 2 * kTcABytes),
                       at<uint32_t>(oTc + 2 * kTcABytes + kTcBBytes), tc_mbar(), *tc_slot()};
     }
-    DEVI QRScratch qr() const { return QRScratch{tau(), piv(), ipiv(), vn1(), vn2(), d(), cbc(), ibc(), col(0), col(1),
+    DEVI QRScratch qr() const { return QRScratch{tau(), piv(), ipiv(), vn1(), vn2(), d(), col(0), col(1),
                          reinterpret_cast<long long*>(col(2)), reinterpret_cast<double*>(col(3)), reinterpret_cast<int*>(col(4))}; }
 };
 
@@ -510,8 +508,8 @@ DEVI cplx ratio_unit(double ar, double ai, cplx en, cplx eo) {
 // a site on their own) and the vectors (1.3 K cycles a block).  Against blocks of four
 // with a DFMA pass (number-conserving) and one barrier per site with every thread
 // keeping its elements (Nambu), M cycles of updates per sweep of a chain: 6x6 Nambu
-// block, L = 40, one CTA per SM 89 -> 13.7; 4x4 Nambu, two CTAs 12.8 -> 5.9; 8x8,
-// L = 40 24.0 -> 9.7; 12x12, L = 50 181 -> 144; 6x6, L = 160, two CTAs 26.2 -> 26.4.
+// block, L = 40, one CTA per SM 89 -> 13.4; 4x4 Nambu, two CTAs 12.8 -> 5.7; 8x8,
+// L = 40 24.0 -> 9.6; 12x12, L = 50 181 -> 137; 6x6, L = 160, two CTAs 26.2 -> 25.6.
 static_assert(Cfg<16>::KB == 8 && Cfg<36>::KB == 8 && Cfg<72>::KB == 8 && Cfg<144>::KB == 8,
               "the lead warp holds the block's 8 x 8 submatrix, two rows per lane");
 
@@ -998,14 +996,8 @@ COLD void measure(Ctx<NMAX> x) {
     for (int k = 0; k < 16; ++k) v[k] = 0.0;
     const int* sxy = s.sxy();
     const int T = blockDim.x;
-    const uint32_t dm = div_magic(n);
-    for (int e = tid; e < n * n; e += T) {
-        const int i = div_by(e, dm), j = e - i * n;
-        const cplx a = G[i * LD + j];                 // Grup(i,j)
-        cplx gc = G[j * LD + i];                      // Grupc(i,j) = G(j,i) - delta_ij
-        if (i == j) gc.x -= 1.0;
-        const cplx dui = cmk(G[i * LD + i].x - 1.0, G[i * LD + i].y);
-        const cplx duj = cmk(G[j * LD + j].x - 1.0, G[j * LD + j].y);
+    // a = Grup(i,j), gc = Grupc(i,j) = G(j,i) - delta_ij, du the diagonal of G - 1
+    auto add = [&](int i, int j, cplx a, cplx gc, cplx dui, cplx duj) {
         const cplx tup = cadd(cmul(dui, duj), cmul(gc, a));   // b-flavour density correlator
         const cplx tud = cmulcj(dui, duj);                     // du_i * dd_j
         v[0] += tup.x;
@@ -1026,6 +1018,37 @@ COLD void measure(Ctx<NMAX> x) {
             v[3] += p.y * sfr;
             v[4] += p.x * dwr;
             v[5] += p.y * dwr;
+        }
+    };
+    if constexpr (Cfg<NMAX>::GG) {
+        // G in L2: a warp takes 8 x 4 elements, so that both orders read whole sectors (8 rows of
+        // 64 bytes and 4 rows of 128; a warp along a row reads its mirror from 32 lines), and the
+        // diagonal comes from shared memory: 12x12, L = 50 12.4 -> 5.9 M cycles a sweep.  Elements past
+        // the edge add zeros.
+        cplx* dg = s.delta();   // rewritten by the next channel's proposals
+        for (int i = tid; i < n; i += T) dg[i] = cmk(G[i * LD + i].x - 1.0, G[i * LD + i].y);
+        __syncthreads();
+        const int lane = tid & 31, nt = (n + 3) >> 2, tiles = ((n + 7) >> 3) * nt;
+        const uint32_t dt = div_magic(nt);
+#pragma unroll 2
+        for (int t = tid >> 5; t < tiles; t += T >> 5) {
+            const int rt = div_by(t, dt);
+            const int i0 = 8 * rt + (lane >> 2), j0 = 4 * (t - rt * nt) + (lane & 3);
+            const int i = min(i0, n - 1), j = min(j0, n - 1);
+            const bool in = i0 < n && j0 < n;
+            const cplx z = cmk(0.0, 0.0), a = G[i * LD + j];
+            cplx gc = G[j * LD + i];
+            gc.x -= i == j ? 1.0 : 0.0;
+            add(i, j, in ? a : z, in ? gc : z, in ? dg[i] : z, in ? dg[j] : z);
+        }
+    } else {
+        const uint32_t dm = div_magic(n);
+        for (int e = tid; e < n * n; e += T) {
+            const int i = div_by(e, dm), j = e - i * n;
+            const cplx a = G[i * LD + j];
+            cplx gc = G[j * LD + i];
+            if (i == j) gc.x -= 1.0;
+            add(i, j, a, gc, cmk(G[i * LD + i].x - 1.0, G[i * LD + i].y), cmk(G[j * LD + j].x - 1.0, G[j * LD + j].y));
         }
     }
     for (int e = tid; e < 3 * n; e += blockDim.x) {   // bonds (x+1,y), (x,y+1), (x-1,y+1) (lattice.f90:98-111)
