@@ -633,7 +633,7 @@ def run_headline(args, rank, world, local):
                            "effective sample, so the ESS/s ratio is the equal-error speed-up",
         },
         "roofline": {"bound": "tensor", "pipe": "fp64",
-                     "limiter": "FP64 dependency latency and barriers (the sweep issues DFMA, no tensor instruction)",
+                     "limiter": "FP64 dependency latency and barriers (decisions and factorisations issue DFMA, products and rank passes FP64 mma)",
                      "kernel": "sweep_kernel<36,0>", "achieved": sweep_tflops, "peak": fp64_peak,
                      "unit": "TFLOP/s", "frac": sweep_tflops / fp64_peak, "traffic": traffic,
                      "traffic_source": "dram bytes of one launch from the ncu capture in "
