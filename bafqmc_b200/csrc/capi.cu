@@ -836,11 +836,9 @@ int bafqmc_net_collect(bafqmc_net* n, bafqmc_handle* h) {
         return fail(BAFQMC_ESTATE, "bafqmc_net_reserve_data has not reserved a set of this handle's chain count");
     if (n->data_used >= n->data_slots) return fail(BAFQMC_ESTATE, "the training set is full");
     CK(cudaSetDevice(h->device));
-    cudaStream_t own = n->stream;
-    n->stream = h->stream;
-    const cudaError_t e = bq::launch_collect(n, h->args(), n->data_used);
-    n->stream = own;
-    CK(e);
+    const bq::NetOnStream on(n, h->stream);
+    CK(on.error);
+    CK(bq::launch_collect(n, h->args(), n->data_used));
     n->data_used += 1;
     return BAFQMC_OK;
 }
@@ -863,8 +861,8 @@ int bafqmc_learned_move(bafqmc_handle* h, bafqmc_net* n, int* accepted, double* 
         n->move_cap = h->nchains;
     }
     // the network's kernels run on the handle's stream for the move
-    cudaStream_t own = n->stream;
-    n->stream = h->stream;
+    const bq::NetOnStream on(n, h->stream);
+    CK(on.error);
     const bq::KernelArgs ka = h->args(), kp = h->args2();
     cudaError_t e = bq::launch_pack_chains(n, ka);
     if (e == cudaSuccess) e = bq::net_forward(n, h->nchains);
@@ -872,7 +870,6 @@ int bafqmc_learned_move(bafqmc_handle* h, bafqmc_net* n, int* accepted, double* 
     if (e == cudaSuccess) e = bq::launch_pack_chains(n, kp);
     if (e == cudaSuccess) e = bq::net_forward(n, h->nchains);
     if (e == cudaSuccess) e = bq::launch_learned_reverse(n, ka, kp, n->d_lqf, n->d_hastings);
-    n->stream = own;
     CK(e);
     for (int c = 0; c < bq::kNumClasses; ++c)
         CK(bq::launch_pre(c, kp, h->d_cls[c], (int)h->cls_list[c].size(), h->stream));

@@ -56,6 +56,7 @@ inline long long act_chain_elems(const NetShape& s, int planes) {
 struct bafqmc_net {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaEvent_t order = nullptr;   // between this stream and that of a handle (bq::NetOnStream)
     bq::NetShape shape{};
     int cap = 0;   // chains the activation buffers hold
     float* d_params = nullptr;   // float32 master copy (flat, the oracle's layout)
@@ -97,6 +98,38 @@ namespace bq {
 
 int net_fail(int code, const std::string& msg);   // sets bafqmc_last_error's message
 int net_ensure_cap(bafqmc_net* n, int chains);     // activation buffers for `chains`
+
+// A scope in which the network's kernels run on a handle's stream.  Neither stream waits for the other
+// by itself (both are non-blocking), and they share the activations, the parameters and the training
+// set: the handle's stream waits on entry for what the network's own still has to do (the clearing of
+// buffers just allocated, a requantisation), and the network's own on exit for what the scope enqueued.
+// A handle's stream under capture takes neither wait, as it cannot depend on work outside its capture.
+class NetOnStream {
+public:
+    NetOnStream(bafqmc_net* n, cudaStream_t st) : n_(n), own_(n->stream), st_(st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        error = cudaStreamIsCapturing(st, &cap);
+        ordered_ = cap == cudaStreamCaptureStatusNone;
+        if (error == cudaSuccess && ordered_) error = pass(own_, st_);
+        n_->stream = st_;
+    }
+    ~NetOnStream() {
+        n_->stream = own_;
+        if (ordered_ && pass(st_, own_) != cudaSuccess) cudaStreamSynchronize(st_);
+    }
+    NetOnStream(const NetOnStream&) = delete;
+    NetOnStream& operator=(const NetOnStream&) = delete;
+    cudaError_t error;   // of the entry
+
+private:
+    cudaError_t pass(cudaStream_t from, cudaStream_t to) {
+        const cudaError_t e = cudaEventRecord(n_->order, from);
+        return e == cudaSuccess ? cudaStreamWaitEvent(to, n_->order, 0) : e;
+    }
+    bafqmc_net* n_;
+    cudaStream_t own_, st_;
+    bool ordered_ = true;
+};
 
 // input pack into x0 (plane-major bf16 with halos) from fields in the confin
 // order: `chains` configurations back to back (float64), the chains of an

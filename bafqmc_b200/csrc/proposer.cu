@@ -822,6 +822,8 @@ int bafqmc_net_create(int Lx, int Ly, int Ltrot, int width, int device, bafqmc_n
     if (cudaSetDevice(device) != cudaSuccess) return bail(bq::net_fail(BAFQMC_ECUDA, "cudaSetDevice"));
     if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(bq::net_fail(BAFQMC_ECUDA, "cudaStreamCreate"));
+    if (cudaEventCreateWithFlags(&n->order, cudaEventDisableTiming) != cudaSuccess)
+        return bail(bq::net_fail(BAFQMC_ECUDA, "cudaEventCreate"));
     const bq::NetShape& s = n->shape;
     const size_t np = sizeof(float) * (size_t)s.nparams;
     long long wt = 0;
@@ -856,6 +858,7 @@ void bafqmc_net_destroy(bafqmc_net* n) {
     for (void* p : ps)
         if (p) cudaFree(p);
     if (n->h_tin) cudaFreeHost(n->h_tin);
+    if (n->order) cudaEventDestroy(n->order);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
 }
