@@ -815,13 +815,15 @@ DEVI void rank_tiles(const Ctx<NMAX>& x, cplx* G, int n, int w, int nw, bool fli
 
 // Start the copy of a slice's fields (both channels) into shared memory: issued before the
 // products or the measurement that precede the slice's updates, which hide its latency.
+// Eight bytes a copy: the fields may be a caller's buffer (bafqmc_sweep_noalloc), which need
+// not be aligned to more than a double.
 template <int NMAX>
 DEVI void stage_fields(const Ctx<NMAX>& x, int slice) {
-    const int ns = x.P().Ns;
-    const double* src = x.phi + (long)slice * ns * 2;
-    for (int i = threadIdx.x; i < ns; i += blockDim.x)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(x.s.fld() + 2 * i)),
-                     "l"(src + 2 * i)
+    const int nf = 2 * x.P().Ns;
+    const double* src = x.phi + (long)slice * nf;
+    for (int i = threadIdx.x; i < nf; i += blockDim.x)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(x.s.fld() + i)),
+                     "l"(src + i)
                      : "memory");
 }
 

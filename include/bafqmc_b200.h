@@ -345,7 +345,7 @@ void* bafqmc_stream(bafqmc_handle* h);
  * in a fixed device array of BAFQMC_NOALLOC_MAX_BYTES that every GPU loading
  * the library holds until exit.  No cudaMalloc/cudaFree is called.
  *   seeds     [nchains] int32, device memory: in = start seeds, out = advanced
- *   phi       [nchains][Ltrot][Ns][2] doubles, device memory: fields, updated
+ *   phi       [nchains][Ltrot][Ns][2] doubles, device memory: fields, updated (aligned as a double)
  *   chain_obs [nchains][BAFQMC_OBS_SCALARS + Lx*Ly] doubles, device memory: the
  *             bin averages, laid out as bafqmc_bin_chain_obs for that point
  *   stream    cudaStream_t to run on (NULL = legacy default stream)
