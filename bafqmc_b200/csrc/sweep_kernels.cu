@@ -815,16 +815,22 @@ DEVI void rank_tiles(const Ctx<NMAX>& x, cplx* G, int n, int w, int nw, bool fli
 
 // Start the copy of a slice's fields (both channels) into shared memory: issued before the
 // products or the measurement that precede the slice's updates, which hide its latency.
-// Eight bytes a copy: the fields may be a caller's buffer (bafqmc_sweep_noalloc), which need
-// not be aligned to more than a double.
+// A site's two values go in one 16-byte copy where the fields start on 16 bytes (every handle's
+// do), in two of eight where a caller's buffer (bafqmc_sweep_noalloc) is aligned to a double only:
+// eight bytes a copy for all took a 3x3 chain's sweep from 0.950 to 0.964 ms, the two forms from
+// 0.958 to 0.962.
 template <int NMAX>
 DEVI void stage_fields(const Ctx<NMAX>& x, int slice) {
-    const int nf = 2 * x.P().Ns;
-    const double* src = x.phi + (long)slice * nf;
-    for (int i = threadIdx.x; i < nf; i += blockDim.x)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(x.s.fld() + i)),
-                     "l"(src + i)
-                     : "memory");
+    const int ns = x.P().Ns;
+    const double* src = x.phi + (long)slice * ns * 2;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(x.s.fld());
+    if (((uintptr_t)x.phi & 15) == 0) {   // then every slice is: it has an even number of doubles
+        for (int i = threadIdx.x; i < ns; i += blockDim.x)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(src + 2 * i) : "memory");
+    } else {
+        for (int i = threadIdx.x; i < 2 * ns; i += blockDim.x)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8 * i), "l"(src + i) : "memory");
+    }
 }
 
 template <int NMAX, bool LEFT, bool PAIR>
