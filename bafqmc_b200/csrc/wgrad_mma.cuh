@@ -20,6 +20,8 @@
 // of g and x, scalar shared-memory operands) took 39 of the 42 ms of the whole gradient,
 // which is now 3.8 ms (4.4 before the upload was threaded).
 #pragma once
+#include <climits>
+
 #include <cuda_bf16.h>
 
 #include "net.h"
@@ -36,8 +38,26 @@ struct WgradMmaArgs {
     int cin, cout;
     float* dw;                // [27][cout][cin]
     float* db;                // [cout]
-    int pairs, per;           // (chain, site) pairs of the batch, pairs per block
+    long long items;          // runs of 32 slices of the batch's (chain, site) pairs
+    int per;                  // runs per block
 };
+
+// How the batch is split over blocks: a pair's slices are runs of kWgRows (the last one short), and a block
+// takes `per` runs in sequence, whole pairs of at most kWgPoints points in all where a pair has fewer than
+// that, kWgPoints points of a longer one.  The chunks go on the grid's x, whose limit (2^31 - 1) a batch that
+// fits the memory does not reach.
+struct WgradSplit {
+    long long items, chunks;
+    int per;
+};
+inline WgradSplit wgrad_split(int L, long long pairs) {
+    WgradSplit w;
+    const int runs = (L + kWgRows - 1) / kWgRows;
+    w.items = pairs * runs;
+    w.per = L < kWgPoints ? kWgPoints / L * runs : kWgPoints / kWgRows;
+    w.chunks = (w.items + w.per - 1) / w.per;
+    return w;
+}
 
 template <int PO, int PI>
 struct WgradCfg {
@@ -68,23 +88,25 @@ DEVI void wg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// grid (9 spatial offsets, chunks of pairs)
+// grid 9 chunks: the nine spatial offsets of a chunk run side by side and share its rows in L2
 template <int PO, int PI>
 __global__ void __launch_bounds__(kWgThreads, 2) wgrad_mma_kernel(WgradMmaArgs a) {
     using C = WgradCfg<PO, PI>;
     __shared__ __align__(128) unsigned char sm[kWgStages * C::kStage];
     const NetShape& s = a.s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int off = blockIdx.x, ob = off / 3 - 1, oc = off % 3 - 1;
-    const int p0 = blockIdx.y * a.per, p1 = min(a.pairs, p0 + a.per);
-    const int ntc = (s.L + kWgRows - 1) / kWgRows, items = (p1 - p0) * ntc;
+    const int off = blockIdx.x % 9, ob = off / 3 - 1, oc = off % 3 - 1;
+    const int ntc = (s.L + kWgRows - 1) / kWgRows;
+    const long long i0 = (long long)(blockIdx.x / 9) * a.per;
+    const int items = (int)min((long long)a.per, a.items - i0);
+    const int p0 = (int)(i0 / ntc), r0 = (int)(i0 - (long long)p0 * ntc);
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
     const long long prow = s.L + 2;   // rows of a plane
 
-    // stage item it (pair p0 + it / ntc, slices 32 (it % ntc) ..) into slot it % kWgStages
+    // stage item it (run r0 + it from the first of pair p0) into slot it % kWgStages
     const auto fill = [&](int it) {
         if (it < items) {
-            const int pr = it / ntc, t0 = (it - pr * ntc) * kWgRows, p = p0 + pr;
+            const int pr = (r0 + it) / ntc, t0 = (r0 + it - pr * ntc) * kWgRows, p = p0 + pr;
             const int b = p / s.Ns, site = p - b * s.Ns, y = site / s.Lx, xx = site - y * s.Lx;
             const int yn = y + ob + (y + ob < 0 ? s.Ly : 0) - (y + ob >= s.Ly ? s.Ly : 0);
             const int xn = xx + oc + (xx + oc < 0 ? s.Lx : 0) - (xx + oc >= s.Lx ? s.Lx : 0);
@@ -196,9 +218,11 @@ inline cudaError_t launch_wgrad_mma(const NetShape& s, int l, int chains, const 
     a.cout = s.cout[l];
     a.dw = dw;
     a.db = db;
-    a.pairs = chains * s.Ns;
-    a.per = kWgPoints / s.L > 1 ? kWgPoints / s.L : 1;
-    const dim3 grid(9, (a.pairs + a.per - 1) / a.per);
+    const WgradSplit w = wgrad_split(s.L, (long long)chains * s.Ns);
+    a.items = w.items;
+    a.per = w.per;
+    if (w.chunks > INT_MAX / 9) return cudaErrorInvalidValue;
+    const unsigned grid = 9u * (unsigned)w.chunks;
     if (s.pout[l] == 8 && s.pin[l] == 8) wgrad_mma_kernel<8, 8><<<grid, kWgThreads, 0, st>>>(a);
     else if (s.pout[l] == 8) wgrad_mma_kernel<8, 2><<<grid, kWgThreads, 0, st>>>(a);
     else wgrad_mma_kernel<2, 8><<<grid, kWgThreads, 0, st>>>(a);
