@@ -88,10 +88,16 @@ struct QRScratch {
     int* ex;          // n   scale exponents of the columns
 };
 
-// Scale 2^e of a column by its largest entry, as an exponent: 0 for a zero or non-finite column.
+// Scale 2^e of a column by its largest entry, as an exponent: that entry to 2^kQrTop (less for one
+// below 2^-680, as 2^-e has to be finite); 0 for a non-finite column.  The largest power that occurs is
+// the cube of a column's norm, b d2 in qr_block, below 2^(3 kQrTop + 14) for 72 rows and above 2^-1000
+// for a square norm above kQrZero: a column is taken as zero once its remaining norm is 2^-653 of its
+// largest entry.
+constexpr int kQrTop = 320;
+constexpr double kQrZero = 0x1p-666;
 DEVI int scale_exponent(double m) {
     const int e = (int)((__double_as_longlong(m) >> 52) & 0x7ff);
-    return (e == 0 || e == 0x7ff) ? 0 : e - 1022;
+    return e == 0x7ff ? 0 : max(e - 1022 - kQrTop, -1000);
 }
 
 // Pivoted QR of A (n x n): (A P) = Q R with ZGEQP3's pivot rule (the column of largest
@@ -111,8 +117,9 @@ DEVI int scale_exponent(double m) {
 // column that the previous step's update left (every step computes the remaining norms
 // exactly, so ZLAQP2's downdating and its recomputation test are not needed), and the
 // product of the unscaled reflector with a column is under way while sqrt and 1/x are.
-// Columns are scaled by powers of two on entry (exact, and reflectors act on rows), so
-// that no sum of squares over- or underflows whatever D has grown to.
+// Columns are scaled by powers of two on entry (exact, and reflectors act on rows), whatever
+// D has grown to, so that no sum of squares or product of norms over- or underflows until a
+// remaining norm is 2^-653 of its column's largest entry (scale_exponent).
 // Rows leave the registers from the top, a block of LPC at a time, so that no step masks
 // them; a branch or a select per row cost more than the arithmetic (3500 cycles a step).
 // Bound: the chain and the issue of a step on the warps that own columns, 1860 cycles at
@@ -188,7 +195,7 @@ DEVI void qr_block(int n, int ld, int kb, int nthr, cplx* A, const QRScratch& s,
         }
         // beta = b = -sign(Re alpha) |column|, d = alpha - b, tau = (b - alpha) / b = -d / b (ZLARFG);
         // the unscaled reflector (d, x) takes conj(tau) / |d|^2 = -conj(d) / (b |d|^2)
-        const bool zero = !(pn > 1.0e-300);
+        const bool zero = !(pn > kQrZero);
         const double y = rsqrt_fast(zero ? 1.0 : pn), nrm = pn * y;
         const double b = alpha.x >= 0.0 ? -nrm : nrm;
         const cplx d = cmk(alpha.x - b, alpha.y);
