@@ -889,10 +889,13 @@ int bafqmc_net_get_params(bafqmc_net* n, float* params) {
 
 int bafqmc_net_set_tensor_cores(bafqmc_net* n, int enable) {
     if (!n) return bq::net_fail(BAFQMC_EARG, "null network");
-    if (enable && !bq::conv_tc_applies(n->shape, 1, false))
-        return bq::net_fail(BAFQMC_EUNSUPPORTED,
-                            "the tensor-core convolution needs width 64, sites a multiple of 4 and Ltrot a multiple of 32");
-    n->use_tc = n->wgrad_tc = enable ? 1 : 0;
+    bool wgrad = false;   // any layer's weight gradient
+    for (int l = 0; l < bq::kNetLayers; ++l) wgrad = wgrad || bq::wgrad_mma_applies(n->shape, l);
+    const bool conv = bq::conv_tc_applies(n->shape, 1, false);
+    if (enable && !conv && !wgrad)
+        return bq::net_fail(BAFQMC_EUNSUPPORTED, "no layer of this network runs on the tensor cores (they need width 64)");
+    n->use_tc = enable && conv ? 1 : 0;
+    n->wgrad_tc = enable ? 1 : 0;
     return BAFQMC_OK;
 }
 

@@ -207,10 +207,13 @@ int bafqmc_global_shift(bafqmc_handle* h, const double* shift, int* accepted);
  * independently of phi).  Parameters are one float32 vector
  * (per layer W[27][cout][cin] then b[cout]; tap k = 3((b+1)3 + (c+1)) + (a+1)
  * for offsets (a, b, c) in (t, y, x)), the layout of the CPU oracle
- * oracle/proposer.py.  With width 64, Lx*Ly a multiple of 4 and Ltrot a
- * multiple of 32, the 64-channel layers run on the tensor cores (tcgen05,
- * operands staged by TMA); bafqmc_net_set_tensor_cores(n, 0) selects the
- * CUDA-core kernels for the same layers (a cross-check).  A network is not
+ * oracle/proposer.py.  With width 64 the
+ * weight gradients run on the tensor cores (mma.sync), and with Lx*Ly a
+ * multiple of 4 and Ltrot a multiple of 32 also the convolutions of every
+ * layer (tcgen05, operands staged by TMA).  bafqmc_net_set_tensor_cores(n, 0)
+ * selects the CUDA-core kernels for both (a cross-check), (n, 1) returns to
+ * the tensor cores wherever they apply, the state a network is created in;
+ * BAFQMC_EUNSUPPORTED if they apply nowhere.  A network is not
  * thread-safe; it runs on its own stream, and on the ensemble's stream inside
  * bafqmc_learned_move and bafqmc_net_collect. */
 typedef struct bafqmc_net bafqmc_net;
