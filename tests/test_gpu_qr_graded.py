@@ -114,3 +114,23 @@ def test_graded_matrix(lib, nmax, n, rows, cols):
         got = Q.conj().T @ (np.ldexp(dr.real, -ec[c]) + 1j * np.ldexp(dr.imag, -ec[c]))
         col = np.ldexp(A[:, c].real, -ec[c]) + 1j * np.ldexp(A[:, c].imag, -ec[c])
         assert np.max(np.abs(got - col)) <= tol * np.linalg.norm(col)
+
+
+@pytest.mark.parametrize("nmax,n", [(16, 16), (36, 36), (72, 36), (72, 72)])
+def test_factors_as_exact_as_lapacks(lib, nmax, n):
+    """Orthogonality of Q and the residual of the product, as means over matrices U D like those of a wrap, at most
+    1.25 times LAPACK's on the same ones: both round the same sums, and a reflector's two scalars to a unit more here."""
+    import scipy.linalg as sl
+    ld, err = np.clongdouble, np.zeros((2, 2))
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    for seed in range(20):
+        rng = np.random.default_rng(seed)
+        A = np.linalg.qr(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))[0] * np.exp(-rng.uniform(0, 20, n))
+        F, Q, d, piv = A.copy(), np.zeros((n, n), dtype=np.complex128), np.zeros(n), np.zeros(n, dtype=np.int32)
+        assert lib.run(nmax, n, p(F), p(Q), p(d), p(piv)) == 0
+        lq, lr, lp = sl.qr(A, pivoting=True)
+        for k, (q, r, pv) in enumerate(((Q.conj().T, np.triu(F) * d[:, None], piv), (lq, lr, lp))):
+            q = q.astype(ld)
+            err[k] += (np.linalg.norm((q.conj().T @ q - np.eye(n)).astype(complex)),
+                       np.linalg.norm(((q @ r.astype(ld) - A[:, pv]) / np.linalg.norm(A[:, pv], axis=0)).astype(complex)))
+    assert np.all(err[0] <= 1.25 * err[1]), err / 20
