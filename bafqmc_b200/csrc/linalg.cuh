@@ -7,7 +7,7 @@
 // (src/number_conserving/src/stabilization.f90:41-190 and
 // src/common/mymats.f90:20-29): ZGEMM, ZTRMM, ZGEQP3 (its pivoting, with exact
 // remaining norms in place of ZLAQP2's downdated ones), ZUNGQR, ZUNMQR, ZTRSM,
-// ZLAPMR/ZLAPMT.  They are written for the sweep's sizes (n <= 64): one CTA
+// ZLAPMR/ZLAPMT.  They are written for the sweep's sizes (n <= 72): one CTA
 // owns one matrix.  The factorisation and the reflector and triangular-solve
 // sequences keep the columns of their operand in registers and reduce with
 // shuffles; divisions are replaced by precomputed reciprocals.

@@ -1,4 +1,4 @@
-// Dense complex FP64 linear algebra for the largest size class (n up to 160),
+// Dense complex FP64 linear algebra for the largest size class (n up to 144),
 // whose matrices live in a per-chain region of global memory because neither
 // the shared memory of one SM (227 KB) nor its register file holds the five
 // n x n complex matrices a chain works on.  While a chain runs, its region
@@ -18,34 +18,33 @@ DEVI double warp_max(double v) {
     return v;
 }
 
-// Overflow-safe 2-norm of column j, rows [r0, n), by one warp (CM: A is stored
-// column-major, element (r, j) at A[j * ld + r]).
-template <bool CM = false>
+// The factorisation works on a column-major copy: element (r, j) at A[j * ld + r], so that a
+// warp's walk of a column is contiguous.
+// Overflow-safe 2-norm of column j, rows [r0, n), by one warp.
 DEVI double warp_colnorm(int n, int ld, const cplx* A, int j, int r0) {
     const int lane = threadIdx.x & 31;
     double m = 0.0;
-    for (int r = r0 + lane; r < n; r += 32) m = fmax(m, fmax(fabs(A[CM ? j * ld + r : r * ld + j].x), fabs(A[CM ? j * ld + r : r * ld + j].y)));
+    for (int r = r0 + lane; r < n; r += 32) m = fmax(m, fmax(fabs(A[j * ld + r].x), fabs(A[j * ld + r].y)));
     m = warp_max(m);
     if (m == 0.0) return 0.0;
     double s = 0.0;
     for (int r = r0 + lane; r < n; r += 32) {
-        const double a = A[CM ? j * ld + r : r * ld + j].x / m, b = A[CM ? j * ld + r : r * ld + j].y / m;
+        const double a = A[j * ld + r].x / m, b = A[j * ld + r].y / m;
         s += a * a + b * b;
     }
     return m * sqrt(warp_sum(s));
 }
 
-template <bool CM = false>
 DEVI double warp_norm(int n, int ld, const cplx* A, int j, int r0) {
     const int lane = threadIdx.x & 31;
     double ss = 0.0;
     for (int r = r0 + lane; r < n; r += 32) {
-        const cplx a = A[CM ? j * ld + r : r * ld + j];
+        const cplx a = A[j * ld + r];
         ss = fma(a.x, a.x, fma(a.y, a.y, ss));
     }
     ss = warp_sum(ss);
     if (!sumsq_unsafe(ss)) return sqrt(ss);
-    return warp_colnorm<CM>(n, ld, A, j, r0);
+    return warp_colnorm(n, ld, A, j, r0);
 }
 
 // C = A B (n x n <= 144, C apart from the operands) on the FP64 tensor pipe, operands in
@@ -223,14 +222,14 @@ COLD void conj_transpose_big(int n, int ld, cplx* A, cplx* S) {
 // pivot column (barrier); the warps update the trailing columns one by one,
 // column pvt from the old column i, with ZLAQP2's norm downdate (barrier);
 // column i takes the reflector and beta, rows above i of columns i and pvt are
-// swapped (barrier).
-template <int RW, bool CM = false>
+// swapped (barrier).  A is column-major, as above.
+template <int RW>
 COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
-#define QA(r, c) A[CM ? (c) * ld + (r) : (r) * ld + (c)]
+#define QA(r, c) A[(c) * ld + (r)]
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, nw = blockDim.x >> 5;
     const double tol3z = 1.0536712127723509e-08;   // sqrt(2^-53), LAPACK's sqrt(dlamch('E'))
     for (int j = wp; j < n; j += nw) {
-        const double v = warp_norm<CM>(n, ld, A, j, 0);
+        const double v = warp_norm(n, ld, A, j, 0);
         if (lane == 0) {
             s.vn1[j] = v;
             s.vn2[j] = v;
@@ -269,7 +268,7 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
         ss = warp_sum(ss);
         const cplx alpha = QA(i, pvt);
         double xn = sqrt(ss);
-        if (sumsq_unsafe(ss)) xn = warp_colnorm<CM>(n, ld, A, pvt, i + 1);
+        if (sumsq_unsafe(ss)) xn = warp_colnorm(n, ld, A, pvt, i + 1);
         cplx tau = cmk(0.0, 0.0), beta = alpha, scl = cmk(0.0, 0.0);
         if (!(xn == 0.0 && alpha.y == 0.0)) {
             const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn * xn);
@@ -333,7 +332,7 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
                 if (recompute) {
                     if (sumsq_unsafe(rest)) {
                         __syncwarp();
-                        nv1 = (i + 1 < n) ? warp_colnorm<CM>(n, ld, A, j, i + 1) : 0.0;
+                        nv1 = (i + 1 < n) ? warp_colnorm(n, ld, A, j, i + 1) : 0.0;
                     } else {
                         nv1 = sqrt(rest);
                     }
@@ -379,8 +378,7 @@ COLD void qrp_big(int n, int ld, cplx* A, QRScratch s) {
     __syncthreads();
     const uint32_t dm = div_magic(n);
     for (int e = tid; e < n * n; e += blockDim.x) {
-        const int q = div_by(e, dm), t = e - q * n;   // consecutive threads walk the storage order
-        const int r = CM ? t : q, c = CM ? q : t;
+        const int c = div_by(e, dm), r = e - c * n;   // consecutive threads walk the storage order
         if (c >= r) {
             const double x = s.vn1[r];
             const cplx a = QA(r, c);

@@ -26,9 +26,9 @@ template <int NMAX> struct Cfg;
 // LD: leading dimension of the shared-memory matrices, odd so that a column
 // walk over 16-byte elements touches all eight bank groups.  MINB: CTAs per SM for the register
 // budget.  GW: the two workspaces live in HBM (after the chain's arena) and
-// only G and U in shared memory.
+// only G and U in shared memory.  GG: G and U in HBM as well, products staged through shared
+// memory, slice products also on the tensor cores (tc.cuh).
 template <> struct Cfg<16> {
-    static constexpr bool TCORE = false;
     static constexpr int THREADS = 128, MAXE = 2, KB = 8, LD = 17, MINB = 4;
     static constexpr bool GW = false, GG = false;
     static constexpr int MQ = 1, MB = 1, MP = 2;
@@ -37,7 +37,6 @@ template <> struct Cfg<16> {
 };
 // N <= 36: two CTAs per SM, all four matrices in shared memory.
 template <> struct Cfg<36> {
-    static constexpr bool TCORE = false;
     static constexpr int THREADS = 256, MAXE = 6, KB = 8, LD = 37, MINB = 2;
     static constexpr bool GW = false, GG = false;
     static constexpr int MQ = 4, MB = 2, MP = 8;
@@ -46,7 +45,6 @@ template <> struct Cfg<36> {
 };
 // N <= 72: G and U in shared memory, the workspaces in HBM (one CTA per SM)
 template <> struct Cfg<72> {
-    static constexpr bool TCORE = false;
     static constexpr int THREADS = 512, MAXE = 11, KB = 8, LD = 73, MINB = 1;
     static constexpr bool GW = true, GG = false;
     static constexpr int MQ = 6, MB = 2, MP = 6;
@@ -61,9 +59,7 @@ template <> struct Cfg<72> {
 // rows per lane (linalg_big.cuh).
 static_assert(kTcPer * 512 >= 144 * kTcKC, "tensor-core staging: elements per thread must cover a chunk");
 template <> struct Cfg<144> {
-    static constexpr bool TCORE = true;   // slice products may run on the tensor cores (tc.cuh)
-    static constexpr int THREADS = 512, MAXE = 41, KB = 8, LD = 145,
-                         MINB = 1;
+    static constexpr int THREADS = 512, MAXE = 41, KB = 8, LD = 145, MINB = 1;
     static constexpr bool GW = true, GG = true;
     static constexpr bool AUG = false;
     static constexpr int RW = 5, SR = 18, SC = 1;
@@ -119,14 +115,13 @@ struct Smem {
     static constexpr size_t oSeed = oAccf + sizeof(int) * NMAX;
     static constexpr size_t oSxy = oSeed + 16;   // site coordinates x | y << 16
     static constexpr size_t oCnt = oSxy + ((sizeof(int) * NMAX + 15) / 16) * 16;   // nacc[2], nc[2], nobs of the sweep
-    // tensor-core staging (classes with Cfg::TCORE): A hi | A lo | B hi | B lo, then
+    // tensor-core staging (classes with Cfg::GG): A hi | A lo | B hi | B lo, then
     // the MMA barrier, the tensor-memory base, the barrier parity and the on flag
-    static constexpr bool TCORE = Cfg<NMAX>::TCORE;
     static constexpr size_t oMs = oCnt + 48;   // per warp, 16 sums over the sweep's measurements
     static constexpr size_t oEnd = oMs + 16 * sizeof(double) * (Cfg<NMAX>::THREADS / 32);
     static constexpr size_t oTc = ((oEnd + 127) / 128) * 128;
     static constexpr size_t oTcBar = oTc + 2 * kTcABytes + 2 * kTcBBytes;
-    static constexpr size_t bytes() { return TCORE ? oTcBar + 32 : oEnd; }
+    static constexpr size_t bytes() { return GG ? oTcBar + 32 : oEnd; }
 
     template <class T>
     static DEVI T* at(size_t off) { return reinterpret_cast<T*>(bq_smem + off); }
@@ -279,17 +274,16 @@ template <int NMAX>
 DEVI void qrp_any(Ctx<NMAX>& x, cplx* A) {
     using C_ = Cfg<NMAX>;
     if constexpr (C_::GG) {
-        // factorised in a column-major copy in S, so each warp's column walk is
-        // contiguous; the operations and their order are those of the row-major call
+        // factorised in a column-major copy in S
         const int n = x.n;
-    const uint32_t dm = div_magic(n);
+        const uint32_t dm = div_magic(n);
         cplx* S = x.S();
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
             const int r = div_by(e, dm), c = e - r * n;
             S[c * C_::LD + r] = A[r * C_::LD + c];
         }
         __syncthreads();
-        qrp_big<C_::RW, true>(n, C_::LD, S, x.s.qr());
+        qrp_big<C_::RW>(n, C_::LD, S, x.s.qr());
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
             const int r = div_by(e, dm), c = e - r * n;
             A[r * C_::LD + c] = S[c * C_::LD + r];
@@ -334,7 +328,7 @@ DEVI void conj_transpose_any(Ctx<NMAX>& x, cplx* A) {
 // barrier's parity bookkeeping is not used again).
 template <int NMAX, bool RIGHT>
 DEVI void slice_mult(Ctx<NMAX>& x, cplx* X, const double* R) {
-    if constexpr (Cfg<NMAX>::TCORE) {
+    if constexpr (Cfg<NMAX>::GG) {
         if (*x.s.tc_on()) {
             if (tc_product(x.n, Cfg<NMAX>::LD, X, R, x.ldr(), RIGHT, x.s.tcb(), x.s.tc_phase(), *x.s.tc_test() != 0,
                            x.s.tc_pending()))
@@ -350,10 +344,10 @@ DEVI void slice_mult(Ctx<NMAX>& x, cplx* X, const double* R) {
 }
 
 // Tensor memory and the MMA barrier of a CTA that runs mixed-precision products
-// (one CTA per SM in the classes with Cfg::TCORE): allocated after set-up, freed at exit.
+// (one CTA per SM in the classes with Cfg::GG): allocated after set-up, freed at exit.
 template <int NMAX>
 DEVI void tc_begin(Ctx<NMAX>& x, const KernelArgs& ka) {
-    if constexpr (Cfg<NMAX>::TCORE) {
+    if constexpr (Cfg<NMAX>::GG) {
         if (threadIdx.x == 0) {
             *x.s.tc_on() = ka.mixed ? 1 : 0;
             *x.s.tc_phase() = 0;
@@ -374,7 +368,7 @@ DEVI void tc_begin(Ctx<NMAX>& x, const KernelArgs& ka) {
 // if it still has not arrived the chain's status gets bit 3.
 template <int NMAX>
 DEVI void tc_end(Ctx<NMAX>& x, const KernelArgs& ka) {
-    if constexpr (Cfg<NMAX>::TCORE) {
+    if constexpr (Cfg<NMAX>::GG) {
         if (ka.mixed) {
             tc_fence_before();
             __syncthreads();
