@@ -44,7 +44,7 @@ DEVI cplx cdiv(cplx a, cplx b) {
     }
 }
 // 1 / x for the serial chains: the approximate reciprocal (measured within 1e-6) and
-// one cubically convergent step of the Newton family, y (1 + e + e^2) with e = 1 - x y
+// one step of Householder's method of cubic order, y (1 + e + e^2) with e = 1 - x y
 // (within 1.01 ulp of 1.0 / x over 2^-100 .. 2^100, measured).  No branch: the
 // compiler's division ends a basic block, and nothing is scheduled across it.
 // x = 0 and infinite x give NaN.
@@ -54,7 +54,7 @@ DEVI double rcp_fast(double x) {
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
-// 1 / sqrt(x) likewise: the approximation and the third-order step
+// 1 / sqrt(x) likewise: the approximation and the same method's cubic step
 // y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2, for normal x > 0 (within 1.27 * 2^-53 relative
 // of the exact value over 2^-200 .. 2^200, measured; the reciprocal within 1.01 * 2^-53).
 DEVI double rsqrt_fast(double x) {

@@ -10,7 +10,7 @@
 // ZLAPMR/ZLAPMT.  They are written for the sweep's sizes (n <= 72): one CTA
 // owns one matrix.  The factorisation and the reflector and triangular-solve
 // sequences keep the columns of their operand in registers and reduce with
-// shuffles; divisions are replaced by precomputed reciprocals.
+// shuffles; their dependent chains take reciprocals instead of divisions.
 #pragma once
 #include "mma64.cuh"
 
@@ -122,9 +122,9 @@ DEVI int scale_exponent(double m) {
 // remaining norm is 2^-653 of its column's largest entry (scale_exponent).
 // Rows leave the registers from the top, a block of LPC at a time, so that no step masks
 // them; a branch or a select per row cost more than the arithmetic (3500 cycles a step).
-// Bound: the chain and the issue of a step on the warps that own columns, 1860 cycles at
-// n = 36 with the second matrix (1460 without, 1075 at n = 16); 139 K -> 67 K cycles for the
-// factorisation.  The version before kept the matrix in shared memory, reduced over eight
+// Bound: the chain and the issue of a step on the warps that own columns, 1930 cycles at
+// n = 36 with the second matrix (1475 without, 1100 at n = 16; 3720 at n = 72, where the
+// registers spill); 131 K -> 69 K cycles for the factorisation.  The version before kept the matrix in shared memory, reduced over eight
 // lanes, downdated the norms and applied the reflectors in a pass of its own: a wrap of a
 // 36-site chain took 560 K cycles with that one and takes 270 K.
 // The per-thread state of the factorisation: its rows of the column of A and of `in`.

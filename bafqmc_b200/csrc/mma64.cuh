@@ -8,8 +8,8 @@
 // cycles of latency against 4 x 8.5 for the same four dependent DFMAs: three
 // accumulators a warp and two warps a scheduler fill it.  The slice products of
 // one sweep against register tiles of DFMAs, M cycles per chain: 64 sites,
-// L = 40 (operand R in L2) 10.1 -> 4.0; 6x6 Nambu block, L = 40 14.4 -> 5.8;
-// 36 sites, L = 160, two CTAs on the SM 6.6 -> 5.2; 16 sites, L = 80 1.03 -> 0.8.
+// L = 40 (operand R in L2) 10.1 -> 4.2; 6x6 Nambu block, L = 40 14.4 -> 6.2;
+// 36 sites, L = 160, two CTAs on the SM 6.6 -> 5.2; 16 sites, L = 80 1.03 -> 0.7.
 #pragma once
 #include <type_traits>
 

@@ -748,7 +748,7 @@ int check_status(bafqmc_net* n) {
 }
 
 // Host configurations (float64, `b` after `a`) to d_tin as float32, through a pinned buffer
-// that the network keeps.  The conversion reads 24 MB for a training batch of 64 x 6x6 x 160
+// that the network keeps.  The conversion reads 11.8 MB for a training batch of 64 x 6x6 x 160
 // and is bound by one core's memory rate, so it is split over threads from 2^18 values on
 // (below, a thread costs more than it saves); a pinned source copies at the link's rate.
 int upload_configs(bafqmc_net* n, int count, const double* a, const double* b) {
@@ -763,7 +763,9 @@ int upload_configs(bafqmc_net* n, int count, const double* a, const double* b) {
         NCK(cudaMallocHost(&n->h_tin, sizeof(float) * need));
         n->tin_cap = need;
     }
-    float* h = n->h_tin;   // free: the call that used it last waited for its copy
+    // free: the call that used it last waited for its copy, or failed after it, and then a copy that still
+    // reads comes before this call's on the stream
+    float* h = n->h_tin;
     const auto convert = [=](long long k0, long long k1) {
         for (long long k = k0; k < std::min(k1, one); ++k) h[k] = (float)a[k];
         for (long long k = std::max(k0, one); k < k1; ++k) h[k] = (float)b[k - one];

@@ -892,7 +892,7 @@ COLD void prop_channel(Ctx<NMAX> x, int ch, int slice) {
     // scheduler alone.  Every CTA of an SM decides on warp 0: their leads share one scheduler,
     // which no pass uses.  Leads spread over the schedulers wait for the other CTAs' mma: a 6x6
     // sweep of two chains an SM 25.7 ms with the pass on two schedulers only, 24.3 on three,
-    // 24.1 here; 4x4 chains, 14 an SM, 20.4 against 18.6 ms.
+    // 24.1 here; 4x4 chains, 14 an SM, 20.4 against 18.3 ms.
     const int rw = (warp & 3) ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;
     constexpr int NRW = NT / 32 * 3 / 4;
     long long nacc = 0;   // accepted proposals, counted by the lead

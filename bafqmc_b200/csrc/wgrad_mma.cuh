@@ -9,16 +9,18 @@
 // offset.  A block takes one spatial offset (b, c), stages 32 slices of g and 34 of x
 // of a (chain, site) pair per step (cp.async, four stages) and accumulates its three
 // time taps from the same rows: 12 m16n8k16 per five ldmatrix.x4 of a warp.  K is split
-// over blocks so that a float32 accumulator takes about 640 points before it is added
+// over blocks so that a float32 accumulator takes at most 640 points before it is added
 // to the result in global memory (the batch has 10^5 to 10^6): the tensor cores truncate
 // where they add, and 2560 points left 3e-6 of the gradient, 640 less than 1e-6 (and are
-// no slower: 3.54 against 3.71 ms for the whole call).
+// no slower: 3.54 against 3.71 ms for the whole call, on one host).
 //
-// Bound: shared-memory reads of the fragments and the mma rate, about 160 and 190 cycles
-// per 16 slices of a block.  64 -> 64 channels, 64 configurations of 6x6 x 160: 0.43 ms a
-// layer (81 GFLOP); the CUDA-core products of one tap per block that it replaces (27 reads
-// of g and x, scalar shared-memory operands) took 39 of the 42 ms of the whole gradient,
-// which is now 3.8 ms (4.4 before the upload was threaded).
+// Bound: issue and latency of 16 warps an SM (registers allow two blocks): issue slots 44%,
+// shared-memory wavefronts 44%, tensor pipe 35% of their peaks.  64 -> 64 channels, 64
+// configurations of 6x6 x 160: 0.44 ms a layer, 81 GFLOP, 0.11 of the measured bf16 peak; the
+// CUDA-core products of one tap per block that it replaces (27 reads of g and x, scalar
+// shared-memory operands) took 39 of the 42 ms of the whole gradient, which is 3.5 to 3.7 ms
+// now, by the host that converts the configurations.  tcgen05 has not been tried: it takes these
+// operands as tiles with K along the rows.
 #pragma once
 #include <climits>
 
