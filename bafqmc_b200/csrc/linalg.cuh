@@ -197,7 +197,7 @@ DEVI void qr_block(int n, int ld, int kb, int nthr, cplx* A, const QRScratch& s,
         // the unscaled reflector (d, x) takes conj(tau) / |d|^2 = -conj(d) / (b |d|^2)
         const bool zero = !(pn > kQrZero);
         const double y = rsqrt_fast(zero ? 1.0 : pn), nr = pn * y;
-        const double nrm = fma(0.5 * y, fma(-nr, nr, pn), nr);   // rounded as sqrt is
+        const double nrm = fma(0.5 * y, fma(-nr, nr, pn), nr);   // a Newton (Heron) step: rounded as sqrt is
         const double b = alpha.x >= 0.0 ? -nrm : nrm;
         const cplx d = cmk(alpha.x - b, alpha.y);
         const double d2 = fma(d.x, d.x, d.y * d.y);

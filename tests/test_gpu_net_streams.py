@@ -88,3 +88,33 @@ def test_training_behind_a_queued_collection(setup):
                 ens.synchronize()
             losses.append(net.train(1, 64, 1, 1e-3, seed=5)[0])
     assert abs(losses[1] - losses[0]) <= 1e-12 * abs(losses[0])
+
+
+def test_move_captured_on_the_handles_stream(setup):
+    """A handle's stream under capture takes no wait on the network's own stream, which is outside the capture."""
+    import ctypes as C
+    ens, params, seeds, phi = setup
+    cu = C.CDLL("libcuda.so.1")
+    stream = C.c_void_p(ens.stream)
+    got = []
+    with _net(params) as net:
+        _start(ens, seeds, phi)
+        ens.learned_move(net)   # allocates
+        for capture in (False, True):
+            _start(ens, seeds, phi)
+            net.status()
+            if capture:
+                graph, run = C.c_void_p(), C.c_void_p()
+                assert cu.cuStreamBeginCapture_v2(stream, 2) == 0   # relaxed
+                ens.learned_move(net, want=False)
+                assert cu.cuStreamEndCapture(stream, C.byref(graph)) == 0
+                assert cu.cuGraphInstantiateWithFlags(C.byref(run), graph, C.c_ulonglong(0)) == 0
+                assert cu.cuGraphLaunch(run, stream) == 0
+            else:
+                ens.learned_move(net, want=False)
+            ens.synchronize()
+            got.append(_state(ens))
+            if capture:
+                assert cu.cuGraphExecDestroy(run) == 0 and cu.cuGraphDestroy(graph) == 0
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
